@@ -281,6 +281,9 @@ struct DevProblem {
         void* gent = nullptr;         // slice-ordered CSR copy (GrpEnt entries)
         int64_t* gptr = nullptr;      // [G][S + 1]
         int32_t *sl_start = nullptr, *sl_key = nullptr, *kslice = nullptr;
+        int NF = 0;                   // pieces (slice x cluster), C > 1
+        int32_t *f_key = nullptr, *f_base = nullptr, *f_kslice = nullptr;
+        int64_t* f_ptr = nullptr;     // [G][NF + 1]
         double* rs = nullptr;
         double* rw = nullptr;
         int32_t* rm = nullptr;
@@ -694,32 +697,54 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
         LAUNCH(launch_group_starts(kout, n, K, gsF, st));
     }
     dbg_mark(ctx, "g.sort");
-    // slices: each key's range cut into pieces of at most kSliceCells cells
+    // slices: each design row's range (its keys are contiguous) cut into
+    // ranges of at most kSliceCells cells, whatever the clusters: the passes
+    // without clusters sum whole design rows.  The clustered bread/meat pass
+    // walks the pieces (slice x cluster): within a design row the cells are in
+    // cluster order, so a gene's entries of a slice are too, and a piece is a
+    // run of them (f_ptr).
     std::vector<int64_t> hks(K + 1);
     CK(cudaMemcpyAsync(hks.data(), kst, (K + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    std::vector<int32_t> sl_start{0}, sl_key, kslice(K + 1);
-    for (int k = 0; k < K; ++k) {
-        kslice[k] = (int32_t)sl_key.size();
-        const int64_t a = hks[k], cnt = hks[k + 1] - hks[k];
-        const int64_t pieces = (cnt + kSliceCells - 1) / kSliceCells;
-        for (int64_t q = 1; q <= pieces; ++q) {
-            sl_start.push_back((int32_t)(a + cnt * q / pieces));
-            sl_key.push_back(k);
+    std::vector<int32_t> sl_start{0}, sl_key, kslice(U + 1);
+    std::vector<int32_t> f_key, f_base, f_slice, f_loc, f_kslice(K + 1);
+    for (int u = 0; u < U; ++u) {
+        kslice[u] = (int32_t)sl_key.size();
+        const int64_t a = hks[u * C], cnt = hks[(u + 1) * C] - a;
+        const int64_t ranges = (cnt + kSliceCells - 1) / kSliceCells;
+        for (int64_t q = 1; q <= ranges; ++q) {
+            sl_start.push_back((int32_t)(a + cnt * q / ranges));
+            sl_key.push_back(u);
         }
     }
-    kslice[K] = (int32_t)sl_key.size();
+    kslice[U] = (int32_t)sl_key.size();
     const int NSL = (int)sl_key.size();
     if (NSL < 1 || NSL > kMaxSlices) {
         if (ctx->debug) fprintf(stderr, "devil_b200: design not grouped (%d slices)\n", NSL);
         return;
     }
+    if (C > 1) {
+        int sl = 0;
+        for (int k = 0; k < K; ++k) {
+            f_kslice[k] = (int32_t)f_key.size();
+            for (int64_t a = hks[k]; a < hks[k + 1];) {
+                while (sl_start[sl + 1] <= a) ++sl;  // (no slice is empty)
+                f_key.push_back(k);
+                f_slice.push_back(sl);
+                f_base.push_back(sl_start[sl]);
+                f_loc.push_back((int32_t)(a - sl_start[sl]));
+                a = std::min<int64_t>(hks[k + 1], sl_start[sl + 1]);
+            }
+        }
+        f_kslice[K] = (int32_t)f_key.size();
+    }
+    const int NF = (int)f_key.size();
     int32_t* d_sl_start = ws<int32_t>(ctx, "grp_sl_start", NSL + 1);
     int32_t* d_sl_key = ws<int32_t>(ctx, "grp_sl_key", NSL);
-    int32_t* d_kslice = ws<int32_t>(ctx, "grp_kslice", K + 1);
+    int32_t* d_kslice = ws<int32_t>(ctx, "grp_kslice", U + 1);
     h2d(ctx, d_sl_start, sl_start.data(), NSL + 1);
     h2d(ctx, d_sl_key, sl_key.data(), NSL);
-    h2d(ctx, d_kslice, kslice.data(), K + 1);
+    h2d(ctx, d_kslice, kslice.data(), U + 1);
     int32_t* cslice = ws<int32_t>(ctx, "grp_cslice", n);
     int32_t* cloc = ws<int32_t>(ctx, "grp_cloc", n);
     double* E = ws<double>(ctx, "grp_E", n);  // exp(offset) in slice order
@@ -751,6 +776,22 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     int32_t* hist = ws<int32_t>(ctx, "grp_hist", (size_t)std::max<int64_t>(nsegs, 1) * NSL);
     LAUNCH(launch_group_csr(dp.rowptr, dp.col, dp.val, dp.val_u16, dp.G, segbase, S, cslice, cloc,
                             NSL, hist, nsegs, gptr, gent, st));
+    if (NF > 0) {
+        auto& gr = dp.grp;
+        auto up = [&](const char* nm, const std::vector<int32_t>& v) {
+            int32_t* d = ws<int32_t>(ctx, nm, v.size());
+            h2d(ctx, d, v.data(), v.size());
+            return d;
+        };
+        gr.f_key = up("grp_f_key", f_key);
+        gr.f_base = up("grp_f_base", f_base);
+        gr.f_kslice = up("grp_f_kslice", f_kslice);
+        int32_t* d_f_slice = up("grp_f_slice", f_slice);
+        int32_t* d_f_loc = up("grp_f_loc", f_loc);
+        gr.NF = NF;
+        gr.f_ptr = ws<int64_t>(ctx, "grp_f_ptr", (size_t)dp.G * (NF + 1));
+        LAUNCH(launch_piece_ptr(gent, dp.val_u16, gptr, dp.G, NSL, d_f_slice, d_f_loc, NF, gr.f_ptr, st));
+    }
     dbg_mark(ctx, "g.csr");
     CK(cudaMemcpyAsync(h + 1, bad + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -932,6 +973,11 @@ GrpGeom grp_geom(const DevProblem& dp) {
     gg.sl_start = gr.sl_start;
     gg.sl_key = gr.sl_key;
     gg.kslice = gr.kslice;
+    gg.NF = gr.NF;
+    gg.f_key = gr.f_key;
+    gg.f_base = gr.f_base;
+    gg.f_kslice = gr.f_kslice;
+    gg.f_ptr = gr.f_ptr;
     gg.rs = gr.rs;
     gg.rw = gr.rw;
     gg.rm = gr.rm;

@@ -155,7 +155,7 @@ template <> struct GrpEnt<float> {
 };
 
 struct GrpGeom {
-    int P, U, C;           // design columns, groups, clusters folded into the keys (1: none)
+    int P, U, C;           // design columns, groups, clusters (1: none) of the bread/meat pass
     int S;                 // slices
     int fine;              // 1: groups are (row, cluster) pairs, one output segment per cluster
     const double* xg;      // [U][P] distinct design rows
@@ -163,8 +163,14 @@ struct GrpGeom {
     const void* gent;      // CSR copy: GrpEnt entries ordered by slice within each gene
     const int64_t* gptr;   // [G][S + 1] absolute start of every slice's entries
     const int32_t* sl_start;  // [S + 1] first cell (slice order) of every slice
-    const int32_t* sl_key;    // [S] its key u * C + c
-    const int32_t* kslice;    // [U*C + 1] first slice of every key (slices ordered by key)
+    const int32_t* sl_key;    // [S] its design row u
+    const int32_t* kslice;    // [U + 1] first slice of every design row (slices ordered by row)
+    // C > 1: the pieces (slice x cluster), ordered by key u * C + cluster
+    int NF;
+    const int32_t* f_key;     // [NF] key
+    const int32_t* f_base;    // [NF] first cell of its slice
+    const int32_t* f_kslice;  // [U*C + 1] first piece of every key
+    const int64_t* f_ptr;     // [G][NF + 1] absolute start of every piece's entries
     double* gsum;          // slice-major IRLS: [slots][S][NQ] per-(gene, slice) sums
     double* rowexp;        // slice-major passes: [G][U] exp(x_u . beta) by gene
     double* psitab;        // slice-major MLE: [slots][kGrpTab] psi tables, psi(a), psi1(a)
@@ -257,6 +263,11 @@ cudaError_t launch_grp_slices(PassKind kind, const GrpGeom& geo, const PassParam
 cudaError_t launch_slice_cells(const int32_t* pnew, const int32_t* sl_start, int S, int64_t n,
                                const double* off, int32_t* cslice, int32_t* cloc, double* E,
                                cudaStream_t st);
+// f_ptr (G x (NF + 1)): each gene's first entry in every piece (the cells of
+// slice[f] from index loc[f] on)
+cudaError_t launch_piece_ptr(const void* gent, int val_u16, const int64_t* gptr, int64_t G, int S,
+                             const int32_t* slice, const int32_t* loc, int NF, int64_t* f_ptr,
+                             cudaStream_t st);
 // beta_0 of a grouped design: geo.act / geo.n_act list every gene, geo.gsum
 // holds G x S doubles; zero_beta is G x P zeros
 cudaError_t launch_grp_init_beta(const GrpGeom& geo, int val_u16, const double* zero_beta,

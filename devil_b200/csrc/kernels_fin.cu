@@ -190,7 +190,7 @@ __global__ void grp_irls_finalize_kernel(GrpGeom geo, int32_t* act_next, int32_t
                                          int32_t* status, int max_iter, double eps,
                                          const float* kf, int8_t* keep) {
     extern __shared__ double fsh[];
-    const int P = geo.P, U = geo.U, C = geo.C, S = geo.S, LD = wla_ld(P);
+    const int P = geo.P, U = geo.U, S = geo.S, LD = wla_ld(P);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // group sums, then H (P x LD) for the LU step, or the compact store of
     // the Schur step (rows of the dense columns, the diagonal) and its
@@ -208,14 +208,14 @@ __global__ void grp_irls_finalize_kernel(GrpGeom geo, int32_t* act_next, int32_t
     const double* gsum = geo.gsum + (int64_t)slot * S * 2;
     // group sums: lanes over slices (one coalesced load each), then a
     // segmented warp scan over each run of slices of one group (a group's
-    // slices are contiguous, keyed u * C + c); the run's last lane adds it in
+    // slices are contiguous); the run's last lane adds it in
     for (int i = lane; i < 2 * U; i += 32) gs[i] = 0.0;
     __syncwarp();
     for (int b = 0; b < S; b += 32) {
         const int sl = b + lane;
         const bool ok = sl < S;
         double v0 = ok ? gsum[sl * 2] : 0.0, v1 = ok ? gsum[sl * 2 + 1] : 0.0;
-        const int q = ok ? __ldg(geo.sl_key + sl) / C : -1 - lane;  // past S: runs of their own
+        const int q = ok ? __ldg(geo.sl_key + sl) : -1 - lane;  // past S: runs of their own
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double t0 = __shfl_up_sync(0xffffffffu, v0, o), t1 = __shfl_up_sync(0xffffffffu, v1, o);

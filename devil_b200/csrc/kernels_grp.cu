@@ -12,11 +12,11 @@
 //     Gauss rule; checked against exact sums before use;
 //   * the corrections of the nonzero counts from a CSR copy in which every
 //     gene's entries are ordered by "slice": the cells are renumbered so
-//     that each (design row, cluster) group is a contiguous range, cut into
-//     slices of at most kSliceCells cells; an entry is 4 bytes (the cell's
-//     16-bit index within its slice and the 16-bit count), and exp(offset)
-//     is stored in the new cell order, so one slice's values fit in shared
-//     memory;
+//     that each design row (and, within it, each cluster) is a contiguous
+//     range, the design rows cut into slices of at most kSliceCells cells;
+//     an entry is 4 bytes (the cell's 16-bit index within its slice and the
+//     16-bit count), and exp(offset) is stored in the new cell order, so one
+//     slice's values fit in shared memory;
 // and assembles the p x p terms from the group sums.  A pass then reads
 // every nonzero once and costs O(nnz + groups x nodes) per gene, plus the
 // assembly over the (group, output) pairs whose design entries are nonzero
@@ -564,8 +564,15 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
     const int slot = blockIdx.x;
     if (slot >= *geo.n_act) return;
     const int g = __ldg(geo.act + slot);
-    const int P = geo.P, U = geo.U, C = geo.C, S = geo.S;
+    const int P = geo.P, U = geo.U, C = geo.C;
     const int NGq = geo.fine ? U * C : U;
+    // fine: the pieces (slice x cluster), keyed u * C + cluster, their cells
+    // counted from the start of their slice; else the slices, keyed u
+    const bool pieces = geo.fine && C > 1;
+    const int S = pieces ? geo.NF : geo.S;
+    const int32_t* skey = pieces ? geo.f_key : geo.sl_key;
+    const int32_t* sbase = pieces ? geo.f_base : geo.sl_start;
+    const int32_t* kfirst = pieces ? geo.f_kslice : geo.kslice;
     extern __shared__ double gsm[];
     double* bet = gsm;                                   // [P]
     double* gs = bet + P;                                // [NGq][NQ] group sums
@@ -588,7 +595,7 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
     }
     const int warp = t >> 5, lane = t & 31, nw = nt >> 5;
     const ET* __restrict__ gent = static_cast<const ET*>(geo.gent);
-    const int64_t* gp = geo.gptr + (int64_t)g * (S + 1);
+    const int64_t* gp = (pieces ? geo.f_ptr : geo.gptr) + (int64_t)g * (S + 1);
     // chunk size grows with the gene's nonzeros so that there are at most
     // S + kGrpUnitsMax nonzero units
     const int64_t CH = max((int64_t)kGrpChunk, (gp[S] - gp[0] + kGrpUnitsMax - 1) / kGrpUnitsMax);
@@ -642,9 +649,9 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
                 sl = lo;
             }
             const int jc = cu - sstart[sl];
-            const int u = __ldg(geo.sl_key + sl) / C;
+            const int u = __ldg(skey + sl) / (pieces ? C : 1);
             const double A = exp(row_dot(geo, u, bet, lane));
-            const double* __restrict__ Es = geo.E + __ldg(geo.sl_start + sl);
+            const double* __restrict__ Es = geo.E + __ldg(sbase + sl);
             const int64_t e0 = __ldg(gp + sl) + jc * CH;
             const int64_t e1 = min(e0 + CH, __ldg(gp + sl + 1));
             // batches of kGrpUnr entries per lane, software-pipelined: the
@@ -693,12 +700,11 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
     }
     __syncthreads();
     // group sums in unit order: the rule unit, then the chunks of the
-    // group's slices (slices are ordered by key u * C + c)
+    // group's slices or pieces (they are ordered by key)
     for (int i = t; i < NGq * NQ; i += nt) {
         const int q = i / NQ, c = i - q * NQ;
         double v = up[q * NQ + c];
-        const int k0 = geo.fine ? q : q * C, k1 = geo.fine ? q + 1 : q * C + C;
-        const int s0 = __ldg(geo.kslice + k0), s1 = __ldg(geo.kslice + k1);
+        const int s0 = __ldg(kfirst + q), s1 = __ldg(kfirst + q + 1);
         for (int un = sstart[s0]; un < sstart[s1]; ++un) v += up[(NGq + un) * NQ + c];
         gs[i] = v;
     }
@@ -842,8 +848,8 @@ __global__ void __launch_bounds__(kSlNT, 1) grp_slices_kernel(GrpGeom geo, typen
             if (i < nc) Es[i] = kInitZ ? log1p(1.0 / e[k]) : e[k];
         }
     }
-    const int u = __ldg(geo.sl_key + s) / geo.C;
-    const bool first = s == __ldg(geo.kslice + u * geo.C);  // the group's rule goes here
+    const int u = __ldg(geo.sl_key + s);
+    const bool first = s == __ldg(geo.kslice + u);  // the group's rule goes here
     constexpr bool kRule = !std::is_same<Pass, PassInitZ>::value;  // zero counts contribute
     const int m = (kRule && first) ? __ldg(geo.rm + u) : 0;
     // the group's rule (node weights, exp(node offsets)) in shared memory:
@@ -1171,14 +1177,14 @@ __global__ void __launch_bounds__(256) grp_assemble_kernel(GrpGeom geo) {
     constexpr int NWV = NW + NV + NF, NS = Pass::NS, NQ = NWV + NS;
     const int slot = blockIdx.x;
     if (slot >= *geo.n_act) return;
-    const int P = geo.P, U = geo.U, C = geo.C, S = geo.S;
+    const int P = geo.P, U = geo.U, S = geo.S;
     extern __shared__ double gs[];  // [U][NQ]
     const int t = threadIdx.x, nt = blockDim.x;
     const double* gsum = geo.gsum + (int64_t)slot * S * NQ;
     for (int i = t; i < U * NQ; i += nt) {
         const int q = i / NQ, c = i - q * NQ;
         double v = 0.0;
-        for (int sl = __ldg(geo.kslice + q * C); sl < __ldg(geo.kslice + q * C + C); ++sl)
+        for (int sl = __ldg(geo.kslice + q); sl < __ldg(geo.kslice + q + 1); ++sl)
             v += gsum[sl * NQ + c];
         gs[i] = v;
     }
@@ -1305,11 +1311,11 @@ __global__ void grp_init_finish_kernel(GrpGeom geo, const double* ginv, int64_t 
     const int64_t g = blockIdx.x;
     if (g >= G) return;
     const int t = threadIdx.x, nt = blockDim.x;
-    const int U = geo.U, C = geo.C, P = geo.P, S = geo.S;
+    const int U = geo.U, P = geo.P, S = geo.S;
     const double* gs = geo.gsum + g * S;
     for (int u = t; u < U; u += nt) {
         double z = 0.0;
-        for (int sl = __ldg(geo.kslice + u * C); sl < __ldg(geo.kslice + u * C + C); ++sl) z += gs[sl];
+        for (int sl = __ldg(geo.kslice + u); sl < __ldg(geo.kslice + u + 1); ++sl) z += gs[sl];
         zu[u] = z;
     }
     __syncthreads();
@@ -1364,7 +1370,7 @@ template <class Pass>
 static cudaError_t grp_run(const GrpGeom& geo, const PassParamsAny& pa, PassKind kind, int val_u16,
                            int max_slots, cudaStream_t st) {
     const int NGq = geo.fine ? geo.U * geo.C : geo.U;
-    const size_t smem = grp_smem_bytes(kind, geo.P, NGq, geo.S);
+    const size_t smem = grp_smem_bytes(kind, geo.P, NGq, geo.fine && geo.C > 1 ? geo.NF : geo.S);
     auto prm = grp_params<Pass>(pa);
     auto go = [&](auto kern) -> cudaError_t {
         // static shared memory (psi tables) counts against the 48 KB default
@@ -1413,6 +1419,47 @@ cudaError_t launch_slice_cells(const int32_t* pnew, const int32_t* sl_start, int
                                cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     slice_cells_kernel<<<nblk(n, 256), 256, 0, st>>>(pnew, sl_start, S, n, off, cslice, cloc, E);
+    return cudaGetLastError();
+}
+
+// f_ptr[g][f]: the first entry of gene g in piece f (a cluster's cells of a
+// slice, starting at index loc[f] of slice[f]); the entries of a slice are in
+// cell order, so a search in the slice's range finds it.  f_ptr[g][NF] is the
+// end of the row.
+template <class VT>
+__global__ void piece_ptr_kernel(const typename GrpEnt<VT>::T* gent, const int64_t* gptr, int64_t G, int S,
+                                 const int32_t* slice, const int32_t* loc, int NF, int64_t* f_ptr) {
+    const int64_t total = G * (NF + 1);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t g = i / (NF + 1);
+        const int f = (int)(i - g * (NF + 1));
+        const int64_t* gp = gptr + g * (S + 1);
+        int64_t lo = gp[S];
+        if (f < NF) {
+            const int sl = __ldg(slice + f), l = __ldg(loc + f);
+            lo = gp[sl];
+            int64_t hi = gp[sl + 1];
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (GrpEnt<VT>::loc(gent[mid]) < l) lo = mid + 1; else hi = mid;
+            }
+        }
+        f_ptr[i] = lo;
+    }
+}
+
+cudaError_t launch_piece_ptr(const void* gent, int val_u16, const int64_t* gptr, int64_t G, int S,
+                             const int32_t* slice, const int32_t* loc, int NF, int64_t* f_ptr,
+                             cudaStream_t st) {
+    if (G <= 0) return cudaSuccess;
+    const unsigned grid = (unsigned)std::min<int64_t>(nblk(G * (NF + 1), 256), 148 * 32);
+    if (val_u16)
+        piece_ptr_kernel<uint16_t><<<grid, 256, 0, st>>>(static_cast<const GrpEnt<uint16_t>::T*>(gent), gptr, G, S,
+                                                         slice, loc, NF, f_ptr);
+    else
+        piece_ptr_kernel<float><<<grid, 256, 0, st>>>(static_cast<const GrpEnt<float>::T*>(gent), gptr, G, S, slice,
+                                                      loc, NF, f_ptr);
     return cudaGetLastError();
 }
 
