@@ -341,7 +341,7 @@ void validate_csr(devil_ctx* ctx, DevProblem& dp) {
     gene_order(ctx, dp);
     int32_t* bad = ws<int32_t>(ctx, "csr_bad", 1);
     CK(cudaMemsetAsync(bad, 0, sizeof(int32_t), ctx->stream));
-    LAUNCH(launch_validate_csr(dp.rowptr, dp.col, dp.G, dp.n, dp.nnz, bad, ctx->stream, dp.gorder));
+    LAUNCH(launch_validate_csr(dp.rowptr, dp.col, dp.G, dp.n, dp.nnz, bad, ctx->stream));
     int32_t h = 0;
     CK(cudaMemcpyAsync(&h, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -506,7 +506,8 @@ void prepare_design(devil_ctx* ctx, DevProblem& dp, const double* X, int P, bool
     dp.fine_ptr = ws<int64_t>(ctx, "fine_ptr", (size_t)dp.G * (nf + 1));
     LAUNCH(launch_segptr(dp.rowptr, dp.col, dp.G, dp.fine_bound, nf + 1, dp.fine_ptr, st));
     dp.stats = ws<double>(ctx, "stats", (size_t)dp.G * 6);
-    LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.n, dp.stats, st, dp.gorder));
+    LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.nnz, dp.n, dp.stats,
+                             ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), st));
     CK(cudaStreamSynchronize(st));  // host copies above must stay valid until here
 }
 
@@ -568,7 +569,7 @@ void compute_offsets(devil_ctx* ctx, DevProblem& dp, int method, const double* s
         CK(cudaMemsetAsync(colsum_u32, 0, n * sizeof(uint32_t), st));
     }
     LAUNCH(launch_colstats(dp.rowptr, dp.col, dp.val, dp.val_u16, dp.G, dp.nnz, colsum, collog,
-                           colcnt, colmin, st, colsum_u32, n));
+                           colcnt, colmin, st, colsum_u32, n, dp.gorder));
     int32_t* err = ws<int32_t>(ctx, "sf_err", 1);
     LAUNCH(launch_sf_finalize(method == DEVIL_SF_NORMED_SUM ? 1 : 2, dp.G, n, colsum, collog, colcnt,
                               colmin, offset, dp.sf, dp.off, dp.off_f, err, st));
@@ -2331,7 +2332,8 @@ int devil_estimate_dispersion(devil_ctx* ctx, const devil_counts* counts,
         DevProblem dp;
         upload_counts(ctx, counts, dp);
         dp.stats = ws<double>(ctx, "stats", (size_t)dp.G * 6);
-        LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.n, dp.stats, ctx->stream));
+        LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.nnz, dp.n, dp.stats,
+                                 ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), ctx->stream));
         upload_offsets(ctx, dp, offset_vector);
         double* th = ws<double>(ctx, "theta0", dp.G);
         float* k = ws<float>(ctx, "k", dp.G);

@@ -172,45 +172,37 @@ cudaError_t launch_x_rowmajor_d(const double* Xcm, int64_t n, int P, int xs, dou
 // stats[g*6 + 0..5] = mean, sample variance (n-1), sum y,
 //                     sum (y-1) y, max y, nnz
 // ------------------------------------------------------------------
-template <class VT>
-__global__ void gene_stats_kernel(const int64_t* rowptr, const VT* val, int64_t G, int64_t n,
-                                  double* stats, const int32_t* order) {
+__global__ void gene_stats_kernel(const int64_t* rowptr, const float* val, int64_t G, int64_t n,
+                                  double* stats) {
     int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (g >= G) return;
-    if (order) g = order[g];
     const int64_t e0 = rowptr[g], e1 = rowptr[g + 1];
-    // Counts that are whole numbers (always for uint16; checked for float):
-    // one pass with exact integer sums of y and y^2 (below 2^64 for any int32
-    // cell count and counts below 2^16) and the variance from the exact
-    // numerator n sum y^2 - (sum y)^2 in 128 bits, so a uint16 and a float
-    // copy of the same counts give the same statistics.  Other float counts:
-    // a second pass over the squared deviations in FP64.
+    // Float counts that are whole numbers: one pass with exact integer sums
+    // of y and y^2 (below 2^64 for any int32 cell count and counts below 2^16)
+    // and the variance from the exact numerator n sum y^2 - (sum y)^2 in 128
+    // bits, so a uint16 (gene_sums_kernel) and a float copy of the same counts
+    // give the same statistics.  Other counts: a second pass over the squared
+    // deviations in FP64.
     unsigned long long s1 = 0, s2 = 0;
     double s = 0.0, mx = 0.0;
     bool whole = true;
     constexpr int U = 4;  // loads in flight per lane
     for (int64_t base = e0 + lane; base < e1; base += 32 * U) {
-        VT raw[U];
+        float raw[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) raw[u] = base + 32 * u < e1 ? __ldg(val + base + 32 * u) : VT(0);
+        for (int u = 0; u < U; ++u) raw[u] = base + 32 * u < e1 ? __ldg(val + base + 32 * u) : 0.f;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const double y = (double)raw[u];
             s += y;
             mx = fmax(mx, y);
-            if constexpr (std::is_same<VT, uint16_t>::value) {
-                const unsigned long long v = (unsigned long long)raw[u];
+            const bool w = y >= 0.0 && y < 65536.0 && y == floor(y);
+            whole = whole && w;
+            if (w) {
+                const unsigned long long v = (unsigned long long)y;
                 s1 += v;
                 s2 += v * v;
-            } else {
-                const bool w = y >= 0.0 && y < 65536.0 && y == floor(y);
-                whole = whole && w;
-                if (w) {
-                    const unsigned long long v = (unsigned long long)y;
-                    s1 += v;
-                    s2 += v * v;
-                }
             }
         }
     }
@@ -259,86 +251,144 @@ __global__ void gene_stats_kernel(const int64_t* rowptr, const VT* val, int64_t 
         o[5] = (double)(e1 - e0);
     }
 }
-// The same statistics for uint16 counts whose array starts on a 16-byte
-// boundary: warp per gene, the row read as 16-byte pieces of eight counts
-// (four pieces in flight per lane), pieces that straddle the row's ends
-// masked, the last piece of the array (which may end past nnz) read count
-// by count.  Exact integer sums, as above.
-__global__ void gene_stats_u16v_kernel(const int64_t* rowptr, const uint16_t* val, int64_t G, int64_t n,
-                                       double* stats, const int32_t* order) {
-    int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// The same statistics for uint16 counts, by spans of the value array instead
+// of by rows: a warp takes `span` consecutive entries, cuts them at the row
+// ends, and adds each row's exact integer sums and maximum to the gene's
+// accumulators with atomics (integers: the order does not matter).  A warp
+// per row took as long as the longest row (a gene seen in most of a million
+// cells: 1,000 dependent rounds, 2.49 ms at 790 M entries); the spans read the
+// array near the memory's rate (0.42 ms).  VEC: the array starts on a 16-byte
+// boundary and is read as 16-byte pieces of eight counts (four in flight per
+// lane), pieces that straddle a row's ends masked, the array's last piece
+// (which may end past nnz) read count by count; otherwise count by count.
+struct GeneSums {
+    unsigned long long s1, s2;  // sum y, sum y^2
+    unsigned mx, pad;
+};
+template <bool VEC>
+__global__ void __launch_bounds__(256) gene_sums_kernel(const int64_t* rowptr, const uint16_t* val, int64_t G,
+                                                        int64_t span, GeneSums* acc) {
     const int lane = threadIdx.x & 31;
-    if (g >= G) return;
-    if (order) g = order[g];
-    const int64_t e0 = rowptr[g], e1 = rowptr[g + 1], nnz = rowptr[G];
-    const int64_t p0 = e0 >> 3, p1 = (e1 + 7) >> 3, pfull = nnz >> 3;
+    const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int64_t nnz = rowptr[G], pfull = nnz >> 3;
+    int64_t a = max(w * span, rowptr[0]);
+    const int64_t b = min((w + 1) * span, nnz);
+    if (a >= b) return;
+    int64_t g = 0, hi = G;  // the last row that starts at or before a
+    while (hi - g > 1) {
+        const int64_t mid = (g + hi) >> 1;
+        if (rowptr[mid] <= a) g = mid; else hi = mid;
+    }
     const uint4* v4 = reinterpret_cast<const uint4*>(val);
-    unsigned long long s1 = 0, s2 = 0;
-    unsigned mx = 0;
-    constexpr int U = 4;
-    for (int64_t base = p0 + lane; base < p1; base += 32 * U) {
-        uint4 pc[U];
+    for (; a < b; ++g) {
+        const int64_t e0 = a, e1 = min(rowptr[g + 1], b);
+        if (e1 <= e0) continue;
+        a = e1;
+        unsigned long long s1 = 0, s2 = 0;
+        unsigned mx = 0, mx2 = 0;  // mx2: two 16-bit maxima
+        constexpr int U = 4;
+        if constexpr (VEC) {
+            const int64_t p1 = (e1 + 7) >> 3;
+            for (int64_t base = (e0 >> 3) + lane; base < p1; base += 32 * U) {
+                uint4 pc[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int64_t pp = base + 32 * u;
-            pc[u] = make_uint4(0, 0, 0, 0);
-            if (pp < p1) {
-                if (pp < pfull) {
-                    pc[u] = __ldg(v4 + pp);
-                } else {
-                    uint16_t h[8];
+                for (int u = 0; u < U; ++u) {
+                    const int64_t pp = base + 32 * u;
+                    pc[u] = make_uint4(0, 0, 0, 0);
+                    if (pp < p1) {
+                        if (pp < pfull) {
+                            pc[u] = __ldg(v4 + pp);
+                        } else {
+                            uint16_t h[8];
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) h[r] = pp * 8 + r < nnz ? val[pp * 8 + r] : (uint16_t)0;
-                    pc[u] = make_uint4(h[0] | (unsigned)h[1] << 16, h[2] | (unsigned)h[3] << 16,
-                                       h[4] | (unsigned)h[5] << 16, h[6] | (unsigned)h[7] << 16);
+                            for (int r = 0; r < 8; ++r) h[r] = pp * 8 + r < nnz ? val[pp * 8 + r] : (uint16_t)0;
+                            pc[u] = make_uint4(h[0] | (unsigned)h[1] << 16, h[2] | (unsigned)h[3] << 16,
+                                               h[4] | (unsigned)h[5] << 16, h[6] | (unsigned)h[7] << 16);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int64_t ea = (base + 32 * u) * 8;
+                    if (ea >= e1) continue;
+                    unsigned wd[4] = {pc[u].x, pc[u].y, pc[u].z, pc[u].w};
+                    if (ea < e0 || ea + 8 > e1) {  // a piece across a row's end: zeros outside
+#pragma unroll
+                        for (int r = 0; r < 8; ++r)
+                            if (ea + r < e0 || ea + r >= e1) wd[r >> 1] &= r & 1 ? 0xffffu : 0xffff0000u;
+                    }
+                    unsigned p = 0;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const unsigned lo = wd[r] & 0xffffu, hi = wd[r] >> 16;
+                        p += lo + hi;
+                        asm("mad.wide.u32 %0, %1, %1, %0;" : "+l"(s2) : "r"(lo));
+                        asm("mad.wide.u32 %0, %1, %1, %0;" : "+l"(s2) : "r"(hi));
+                        mx2 = __vmaxu2(mx2, wd[r]);
+                    }
+                    s1 += p;
                 }
             }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int64_t pp = base + 32 * u;
-            if (pp >= p1) continue;
-            const int64_t ea = pp * 8;
-            const unsigned w[4] = {pc[u].x, pc[u].y, pc[u].z, pc[u].w};
-            const bool whole = ea >= e0 && ea + 8 <= e1;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const unsigned y = (w[r >> 1] >> (16 * (r & 1))) & 0xffffu;
-                if (whole || (ea + r >= e0 && ea + r < e1)) {
-                    s1 += y;
-                    s2 += (unsigned long long)(y * y);
-                    mx = max(mx, y);
-                }
+        } else {
+            for (int64_t e = e0 + lane; e < e1; e += 32) {
+                const unsigned y = val[e];
+                s1 += y;
+                s2 += (unsigned long long)(y * y);
+                mx = max(mx, y);
             }
         }
-    }
+        mx = max(mx, max(mx2 & 0xffffu, mx2 >> 16));
 #pragma unroll
-    for (int sh = 16; sh > 0; sh >>= 1) {
-        s1 += __shfl_xor_sync(0xffffffffu, s1, sh);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, sh);
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
-    }
-    if (lane == 0) {
-        double* o = stats + g * 6;
-        const __int128 num = (__int128)n * (__int128)s2 - (__int128)s1 * (__int128)s1;
-        o[0] = (double)s1 / (double)n;
-        o[1] = (double)num / ((double)n * (double)(n - 1));
-        o[2] = (double)s1;
-        o[3] = (double)(s2 - s1);
-        o[4] = (double)mx;
-        o[5] = (double)(e1 - e0);
+        for (int sh = 16; sh > 0; sh >>= 1) {
+            s1 += __shfl_xor_sync(0xffffffffu, s1, sh);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, sh);
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
+        }
+        if (lane == 0) {
+            atomicAdd(&acc[g].s1, s1);
+            atomicAdd(&acc[g].s2, s2);
+            atomicMax(&acc[g].mx, mx);
+        }
     }
 }
+__global__ void gene_stats_from_sums_kernel(const int64_t* rowptr, const GeneSums* acc, int64_t G, int64_t n,
+                                            double* stats) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= G) return;
+    const GeneSums a = acc[g];
+    double* o = stats + g * 6;
+    const __int128 num = (__int128)n * (__int128)a.s2 - (__int128)a.s1 * (__int128)a.s1;
+    o[0] = (double)a.s1 / (double)n;
+    o[1] = (double)num / ((double)n * (double)(n - 1));
+    o[2] = (double)a.s1;
+    o[3] = (double)(a.s2 - a.s1);
+    o[4] = (double)a.mx;
+    o[5] = (double)(rowptr[g + 1] - rowptr[g]);
+}
 
-cudaError_t launch_gene_stats(const int64_t* rowptr, const void* val, int val_u16, int64_t G,
-                              int64_t n, double* stats, cudaStream_t st, const int32_t* order) {
+size_t gene_sums_bytes(int64_t G) { return (size_t)G * sizeof(GeneSums); }
+
+cudaError_t launch_gene_stats(const int64_t* rowptr, const void* val, int val_u16, int64_t G, int64_t nnz,
+                              int64_t n, double* stats, void* sums, cudaStream_t st) {
     if (G == 0) return cudaSuccess;
-    if (val_u16 && (reinterpret_cast<uintptr_t>(val) & 15) == 0)
-        gene_stats_u16v_kernel<<<nblk(G, 8), 256, 0, st>>>(rowptr, (const uint16_t*)val, G, n, stats, order);
-    else if (val_u16)
-        gene_stats_kernel<uint16_t><<<nblk(G, 8), 256, 0, st>>>(rowptr, (const uint16_t*)val, G, n, stats, order);
-    else
-        gene_stats_kernel<float><<<nblk(G, 8), 256, 0, st>>>(rowptr, (const float*)val, G, n, stats, order);
+    if (!val_u16) {
+        gene_stats_kernel<<<nblk(G, 8), 256, 0, st>>>(rowptr, (const float*)val, G, n, stats);
+        return cudaGetLastError();
+    }
+    GeneSums* acc = static_cast<GeneSums*>(sums);
+    cudaError_t e = cudaMemsetAsync(acc, 0, gene_sums_bytes(G), st);
+    if (e != cudaSuccess) return e;
+    // about 64 warps per SM in flight, 1,024 to 16,384 entries each
+    int64_t span = (nnz / (148 * 64) + 255) / 256 * 256;
+    span = std::max<int64_t>(1024, std::min<int64_t>(16384, span));
+    const unsigned b = nblk((nnz + span - 1) / span, 8);
+    if (b > 0) {
+        if ((reinterpret_cast<uintptr_t>(val) & 15) == 0)
+            gene_sums_kernel<true><<<b, 256, 0, st>>>(rowptr, (const uint16_t*)val, G, span, acc);
+        else
+            gene_sums_kernel<false><<<b, 256, 0, st>>>(rowptr, (const uint16_t*)val, G, span, acc);
+    }
+    gene_stats_from_sums_kernel<<<nblk(G, 256), 256, 0, st>>>(rowptr, acc, G, n, stats);
     return cudaGetLastError();
 }
 
@@ -383,10 +433,96 @@ __global__ void colstats_kernel(const int32_t* col, const VT* val, int64_t nnz, 
         }
     }
 }
-// normed_sum column sums of 16-bit counts as 32-bit integer atomics (a
-// column sum is at most G x 65535, below 2^32 for G <= 65537), four entries'
-// loads in flight per thread; colsum_from_u32_kernel turns them into FP64
-// (the same exact integers the FP64 atomics give)
+// normed_sum column sums of 16-bit counts as 32-bit integers (a column sum is
+// at most G x 65535, below 2^32 for G <= 65537); colsum_from_u32_kernel turns
+// them into FP64 (the same exact integers the FP64 atomics give).
+//
+// Columns with many entries: a block keeps kColTile columns' counters in
+// shared memory and takes a share of the genes (blockIdx.y); a gene's entries
+// of the columns are one run of its row (found by a search per lane, 32 genes
+// at a time), read as 16-byte pieces of four cell indices and 8-byte pieces of
+// their counts.  The counters are added to the global ones at the end.
+// Bound by the read (6 B an entry) and the shared atomics' bank conflicts;
+// one global atomic per entry ran at the L2's atomic rate (790 M entries:
+// 2.51 -> 1.17 ms).  (Entries before rowptr[0], which no row holds, are
+// counted too, as the per-entry kernels do.)
+constexpr int kColTile = 49152;  // 192 KB of counters, one block per SM
+__global__ void __launch_bounds__(1024, 1) colsum_tile_kernel(const int64_t* rowptr, const int32_t* col,
+                                                              const uint16_t* val, int64_t G, int64_t n,
+                                                              const int32_t* order, uint32_t* colsum) {
+    extern __shared__ uint32_t ccnt[];
+    const int c0 = blockIdx.x * kColTile;
+    const int c1 = (int)(n - c0 < kColTile ? n : c0 + kColTile);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
+    for (int i = t; i < c1 - c0; i += blockDim.x) ccnt[i] = 0;
+    __syncthreads();
+    const int64_t nnz = rowptr[G], pfull = nnz >> 2;
+    const int4* c4 = reinterpret_cast<const int4*>(col);
+    const uint2* v4 = reinterpret_cast<const uint2*>(val);
+    if (blockIdx.y == 0)
+        for (int64_t e = t; e < rowptr[0]; e += blockDim.x) {
+            const int c = col[e];
+            if (c >= c0 && c < c1) atomicAdd(&ccnt[c - c0], (uint32_t)val[e]);
+        }
+    // warp `w` of the column tile's gridDim.y blocks takes every W-th batch
+    const int64_t W = (int64_t)gridDim.y * nw, w0 = (int64_t)warp * gridDim.y + blockIdx.y;
+    // the genes of a batch are W apart in the list, so that every warp gets a
+    // like share of a list in decreasing order of entries
+    for (int64_t b = 0; b * 32 * W < G; ++b) {
+        const int64_t k = (b * 32 + lane) * W + w0;
+        int64_t lo = 0, hi = 0;
+        if (k < G) {
+            const int64_t g = order ? order[k] : k;
+            const int64_t r0 = rowptr[g], r1 = rowptr[g + 1];
+            auto first_at = [&](int key) {
+                int64_t x = r0, y = r1;
+                while (x < y) {
+                    const int64_t m = (x + y) >> 1;
+                    if (col[m] < key) x = m + 1; else y = m;
+                }
+                return x;
+            };
+            lo = c0 == 0 ? r0 : first_at(c0);
+            hi = c1 >= n ? r1 : first_at(c1);
+        }
+        for (int q = 0; q < 32; ++q) {
+            const int64_t e0 = __shfl_sync(0xffffffffu, lo, q), e1 = __shfl_sync(0xffffffffu, hi, q);
+            const int64_t p1 = (e1 + 3) >> 2;
+            constexpr int U = 4;
+            for (int64_t base = (e0 >> 2) + lane; base < p1 && e0 < e1; base += 32 * U) {
+                int4 c[U];
+                uint2 v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int64_t pp = base + 32 * u;
+                    if (pp < p1 && pp < pfull) {
+                        c[u] = __ldg(c4 + pp);
+                        v[u] = __ldg(v4 + pp);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int64_t pp = base + 32 * u;
+                    if (pp >= p1) continue;
+                    if (pp >= pfull) {  // the array's last piece
+                        for (int64_t e = max(pp * 4, e0); e < e1; ++e) atomicAdd(&ccnt[col[e] - c0], (uint32_t)val[e]);
+                        continue;
+                    }
+                    const int cc[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
+                    const unsigned vv[4] = {v[u].x & 0xffffu, v[u].x >> 16, v[u].y & 0xffffu, v[u].y >> 16};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (pp * 4 + r >= e0 && pp * 4 + r < e1) atomicAdd(&ccnt[cc[r] - c0], vv[r]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < c1 - c0; i += blockDim.x)
+        if (ccnt[i]) atomicAdd(colsum + c0 + i, ccnt[i]);
+}
+// Otherwise: one global atomic per entry, four entries' loads in flight per
+// thread
 __global__ void colsum_u32_kernel(const int32_t* col, const uint16_t* val, int64_t nnz, uint32_t* colsum) {
     constexpr int U = 4;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -412,12 +548,27 @@ __global__ void colsum_from_u32_kernel(const uint32_t* in, int64_t n, double* ou
 cudaError_t launch_colstats(const int64_t* rowptr, const int32_t* col, const void* val,
                             int val_u16, int64_t G, int64_t nnz, double* colsum,
                             double* collog, int32_t* colcnt, int32_t* colmin_bits,
-                            cudaStream_t st, uint32_t* colsum_u32, int64_t n) {
-    (void)rowptr;
+                            cudaStream_t st, uint32_t* colsum_u32, int64_t n, const int32_t* order) {
     if (nnz == 0) return cudaSuccess;
     unsigned b = (unsigned)std::min<int64_t>(nblk(nnz, 256), 148 * 32);
     if (colsum_u32 && val_u16 && !collog && G <= 65537) {
-        colsum_u32_kernel<<<b, 256, 0, st>>>(col, (const uint16_t*)val, nnz, colsum_u32);
+        // the tiles add up to gy counters per column to the global ones: at
+        // most one per eight entries, and a block's SM takes 0.22 ns an entry
+        // against 3.2 ps for the per-entry kernel on the whole chip, so the
+        // tiles pay from 69 blocks on (3.5 M entries in 20,000 columns allow 21
+        // blocks: 71 us against 44 us)
+        const int64_t tiles = (n + kColTile - 1) / kColTile;
+        const int64_t gy = std::min<int64_t>(std::max<int64_t>(1, 148 / tiles), nnz / (8 * n));
+        const bool aligned = (reinterpret_cast<uintptr_t>(col) & 15) == 0 && (reinterpret_cast<uintptr_t>(val) & 7) == 0;
+        if (gy >= 1 && aligned && tiles * gy >= 96) {
+            const size_t smem = (size_t)std::min<int64_t>(n, kColTile) * sizeof(uint32_t);
+            cudaError_t e = raise_dyn_smem(colsum_tile_kernel, (size_t)kColTile * sizeof(uint32_t));
+            if (e != cudaSuccess) return e;
+            colsum_tile_kernel<<<dim3((unsigned)tiles, (unsigned)gy), 1024, smem, st>>>(
+                rowptr, col, (const uint16_t*)val, G, n, order, colsum_u32);
+        } else {
+            colsum_u32_kernel<<<b, 256, 0, st>>>(col, (const uint16_t*)val, nnz, colsum_u32);
+        }
         colsum_from_u32_kernel<<<(unsigned)std::min<int64_t>(nblk(n, 256), 1024), 256, 0, st>>>(colsum_u32, n,
                                                                                                colsum);
         return cudaGetLastError();
@@ -751,102 +902,94 @@ cudaError_t launch_segptr(const int64_t* rowptr, const int32_t* col, int64_t G,
     return cudaGetLastError();
 }
 
-// CSR sanity (warp per gene): rowptr non-decreasing, cell indices in
-// [0, n) and strictly increasing within each row.  bad[0] != 0 on failure.
-__global__ void validate_csr_kernel(const int64_t* rowptr, const int32_t* col, int64_t G, int64_t n,
-                                    int64_t nnz, int32_t* bad, const int32_t* order) {
-    int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    int lane = threadIdx.x & 31;
-    if (g >= G) return;
-    if (order) g = order[g];
-    const int64_t e0 = rowptr[g], e1 = rowptr[g + 1];
-    int b = 0;
-    if (e0 < 0 || e1 < e0 || e1 > nnz) {
-        b = 1;
-    } else {
-        for (int64_t e = e0 + lane; e < e1; e += 32) {
-            int c = col[e];
-            if (c < 0 || c >= n) b = 1;
-            if (e > e0 && col[e - 1] >= c) b = 1;
-        }
-    }
-    b = __any_sync(0xffffffffu, b);
-    if (lane == 0 && b) atomicOr(bad, 1);
-    if (g == G - 1 && lane == 0 && e1 != nnz) atomicOr(bad, 1);
-}
-// The same checks for a cell-index array that starts on a 16-byte boundary:
-// the row read as 16-byte pieces of four indices (four in flight per lane),
-// each index compared with the one before it in the row (the previous
-// piece's last index comes from the lane before, or from the previous
-// round's last lane); the array's last piece, which may end past nnz, is
-// read index by index.
-__global__ void validate_csr_v_kernel(const int64_t* rowptr, const int32_t* col, int64_t G, int64_t n,
-                                      int64_t nnz, int32_t* bad, const int32_t* order) {
-    int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// CSR sanity: row pointers non-decreasing and ending at nnz, cell indices in
+// [0, n) and strictly increasing within each row.  *bad != 0 on failure.  The
+// index array is scanned as one run: an index that does not exceed the one
+// before it must start a row, which a search of the row pointers settles (one
+// per row at most in valid input).  A warp per row took as long as the longest
+// row (2.91 ms at 790 M entries); the scan takes 0.71 ms.
+// VEC: the array starts on a 16-byte boundary and is read as 16-byte pieces of
+// four indices, eight in flight per lane, the index before a piece taken from
+// the lane before (lane 0 loads it); the array's last piece, which may end past
+// nnz, is read index by index.
+template <bool VEC>
+__global__ void __launch_bounds__(256) validate_csr_kernel(const int64_t* rowptr, const int32_t* col, int64_t G,
+                                                           int64_t n, int64_t nnz, int32_t* bad) {
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    if (g >= G) return;
-    if (order) g = order[g];
-    const int64_t e0 = rowptr[g], e1 = rowptr[g + 1];
     int b = 0;
-    if (e0 < 0 || e1 < e0 || e1 > nnz) {
-        b = 1;
-    } else {
-        const int64_t p0 = e0 >> 2, p1 = (e1 + 3) >> 2, pfull = nnz >> 2;
+    for (int64_t g = tid; g < G; g += nt) {
+        const int64_t e0 = rowptr[g], e1 = rowptr[g + 1];
+        if (e0 < 0 || e1 < e0 || e1 > nnz || (g == G - 1 && e1 != nnz)) b = 1;
+    }
+    const int64_t first = max((int64_t)0, min(rowptr[0], nnz));
+    auto starts_row = [&](int64_t e) {
+        int64_t lo = 0, hi = G;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (rowptr[mid] < e) lo = mid + 1; else hi = mid;
+        }
+        return rowptr[lo] == e;
+    };
+    auto check = [&](int64_t e, int before, int c) {
+        if (c < 0 || c >= n) b = 1;
+        if (e > first && before >= c && !starts_row(e)) b = 1;
+    };
+    if constexpr (VEC) {
+        const int64_t p0 = first >> 2, p1 = (nnz + 3) >> 2, pfull = nnz >> 2;
         const int4* c4 = reinterpret_cast<const int4*>(col);
-        constexpr int U = 4;
-        int carry = -1;  // the last index of the previous round (-1: none; indices are >= 0)
-        for (int64_t base = p0; base < p1; base += 32 * U) {
+        constexpr int U = 8;
+        // (whole warps go round together: the shuffles need every lane)
+        for (int64_t base = p0 + (tid - lane); base < p1; base += nt * U) {
             int4 pc[U];
+            int before[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int64_t pp = base + 32 * u + lane;
-                pc[u] = make_int4(-1, -1, -1, -1);
+                const int64_t pp = base + nt * u + lane;
+                pc[u] = make_int4(0, 0, 0, 0);
+                before[u] = -1;
                 if (pp < p1) {
                     if (pp < pfull) {
                         pc[u] = __ldg(c4 + pp);
                     } else {
                         int h[4];
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) h[r] = pp * 4 + r < nnz ? col[pp * 4 + r] : -1;
+                        for (int r = 0; r < 4; ++r) h[r] = pp * 4 + r < nnz ? col[pp * 4 + r] : 0;
                         pc[u] = make_int4(h[0], h[1], h[2], h[3]);
                     }
+                    if (lane == 0 && pp > 0) before[u] = __ldg(col + pp * 4 - 1);
                 }
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int64_t pp = base + 32 * u + lane;
-                // the index before this piece: the previous lane's last, or
-                // (lane 0) the last of round u - 1, or of the previous round
-                int before = __shfl_up_sync(0xffffffffu, pc[u].w, 1);
-                const int last_prev = u > 0 ? __shfl_sync(0xffffffffu, pc[u > 0 ? u - 1 : 0].w, 31) : carry;
-                if (lane == 0) before = last_prev;
-                if (pp < p1) {
-                    const int c[4] = {pc[u].x, pc[u].y, pc[u].z, pc[u].w};
+                const int64_t e = (base + nt * u + lane) * 4;
+                const int up = __shfl_up_sync(0xffffffffu, pc[u].w, 1);
+                if (lane > 0) before[u] = up;
+                // a piece inside the scan that rises from the index before it
+                // (0 or more) to below n is fine: one test for four entries
+                if (before[u] >= 0 && e > first && pc[u].x > before[u] && pc[u].y > pc[u].x && pc[u].z > pc[u].y &&
+                    pc[u].w > pc[u].z && pc[u].w < n)
+                    continue;
+                const int c[5] = {before[u], pc[u].x, pc[u].y, pc[u].z, pc[u].w};
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const int64_t e = pp * 4 + r;
-                        if (e >= e0 && e < e1) {
-                            if (c[r] < 0 || c[r] >= n) b = 1;
-                            const int prv = r == 0 ? before : c[r - 1];
-                            if (e > e0 && prv >= c[r]) b = 1;
-                        }
-                    }
-                }
+                for (int r = 0; r < 4; ++r)
+                    if (e + r >= first && e + r < nnz) check(e + r, c[r], c[r + 1]);
             }
-            carry = __shfl_sync(0xffffffffu, pc[U - 1].w, 31);
         }
+    } else {
+        for (int64_t e = first + tid; e < nnz; e += nt) check(e, e > first ? col[e - 1] : -1, col[e]);
     }
-    b = __any_sync(0xffffffffu, b);
-    if (lane == 0 && b) atomicOr(bad, 1);
-    if (g == G - 1 && lane == 0 && e1 != nnz) atomicOr(bad, 1);
+    if (b) atomicOr(bad, 1);
 }
 cudaError_t launch_validate_csr(const int64_t* rowptr, const int32_t* col, int64_t G, int64_t n,
-                                int64_t nnz, int32_t* bad, cudaStream_t st, const int32_t* order) {
+                                int64_t nnz, int32_t* bad, cudaStream_t st) {
     if (G == 0) return cudaSuccess;
-    if ((reinterpret_cast<uintptr_t>(col) & 15) == 0)
-        validate_csr_v_kernel<<<nblk(G, 8), 256, 0, st>>>(rowptr, col, G, n, nnz, bad, order);
+    const bool vec = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
+    const unsigned b = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nblk(std::max(nnz / 16, G), 256), 148 * 8));
+    if (vec)
+        validate_csr_kernel<true><<<b, 256, 0, st>>>(rowptr, col, G, n, nnz, bad);
     else
-        validate_csr_kernel<<<nblk(G, 8), 256, 0, st>>>(rowptr, col, G, n, nnz, bad, order);
+        validate_csr_kernel<false><<<b, 256, 0, st>>>(rowptr, col, G, n, nnz, bad);
     return cudaGetLastError();
 }
 
