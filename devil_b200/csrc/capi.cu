@@ -474,7 +474,7 @@ void use_device_counts(devil_ctx* ctx, const devil_counts* c, DevProblem& dp) {
     validate_csr(ctx, dp);
 }
 
-// design, segmentation, statistics
+// design and gene statistics
 void prepare_design(devil_ctx* ctx, DevProblem& dp, const double* X, int P, bool X_on_device) {
     if (P < 1 || P > 32) fail(ctx, DEVIL_ERR_UNSUPPORTED, "p = %d outside 1..32", P);
     if (dp.n <= P) fail(ctx, DEVIL_ERR_ARG, "need more cells than design columns");
@@ -488,6 +488,18 @@ void prepare_design(devil_ctx* ctx, DevProblem& dp, const double* X, int P, bool
         h2d(ctx, xd, X, (size_t)dp.n * P);
         dp.Xcm = xd;
     }
+    dp.stats = ws<double>(ctx, "stats", (size_t)dp.G * 6);
+    LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.nnz, dp.n, dp.stats,
+                             ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), st));
+}
+
+// what the per-cell engines read besides the counts: the design by cell and
+// every gene's entries by cell chunk.  A grouped design needs neither (0.9 ms
+// of a 112 ms fit of 10,000 genes x 1 M cells).
+void prepare_cells(devil_ctx* ctx, DevProblem& dp) {
+    if (dp.Xrm) return;
+    const int P = dp.P;
+    cudaStream_t st = ctx->stream;
     // 16 padding rows: TMA copies of the last chunk round up to 4 cells
     dp.Xrm = ws<float>(ctx, "Xrm", (size_t)(dp.n + 16) * dp.xs);
     CK(cudaMemsetAsync(dp.Xrm + (size_t)dp.n * dp.xs, 0, (size_t)16 * dp.xs * sizeof(float), st));
@@ -505,9 +517,6 @@ void prepare_design(devil_ctx* ctx, DevProblem& dp, const double* X, int P, bool
     h2d(ctx, dp.fine_bound, hb.data(), nf + 1);
     dp.fine_ptr = ws<int64_t>(ctx, "fine_ptr", (size_t)dp.G * (nf + 1));
     LAUNCH(launch_segptr(dp.rowptr, dp.col, dp.G, dp.fine_bound, nf + 1, dp.fine_ptr, st));
-    dp.stats = ws<double>(ctx, "stats", (size_t)dp.G * 6);
-    LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.nnz, dp.n, dp.stats,
-                             ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), st));
     CK(cudaStreamSynchronize(st));  // host copies above must stay valid until here
 }
 
@@ -572,7 +581,7 @@ void compute_offsets(devil_ctx* ctx, DevProblem& dp, int method, const double* s
                            colcnt, colmin, st, colsum_u32, n, dp.gorder));
     int32_t* err = ws<int32_t>(ctx, "sf_err", 1);
     LAUNCH(launch_sf_finalize(method == DEVIL_SF_NORMED_SUM ? 1 : 2, dp.G, n, colsum, collog, colcnt,
-                              colmin, offset, dp.sf, dp.off, dp.off_f, err, st));
+                              colmin, offset, dp.sf, dp.off, dp.off_f, ws<double>(ctx, "sf_gm", 1), err, st));
     int32_t herr = 0;
     CK(cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -589,7 +598,8 @@ void compute_offsets(devil_ctx* ctx, DevProblem& dp, int method, const double* s
 // than the cells; otherwise, or when a rule fails its check, the passes
 // stay on the per-cell engines.
 // ------------------------------------------------------------------
-void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int n_clusters, int form) {
+void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int n_clusters, int form,
+                  int overdispersion) {
     dp.grp = DevProblem::Groups{};
     if (form != DEVIL_FORM_CHOSEN || !ctx->use_groups || dp.G == 0) return;
     if (n_clusters > 1 && !ends_host) fail(ctx, DEVIL_ERR_ARG, "cluster_ends is NULL");
@@ -704,18 +714,26 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     // walks the pieces (slice x cluster): within a design row the cells are in
     // cluster order, so a gene's entries of a slice are too, and a piece is a
     // run of them (f_ptr).
+    // A fit with the MLE dispersion cuts at the clusters too.  Its Newton search
+    // resolves the last bracket at rounding level, so sums in another order move
+    // theta by up to 1e-7 on a few genes in 10,000 (beta by 1e-15): fits of one
+    // data set would no longer repeat those of earlier builds to 1e-9.
     std::vector<int64_t> hks(K + 1);
     CK(cudaMemcpyAsync(hks.data(), kst, (K + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    const bool by_cluster = overdispersion == DEVIL_OD_MLE;
     std::vector<int32_t> sl_start{0}, sl_key, kslice(U + 1);
     std::vector<int32_t> f_key, f_base, f_slice, f_loc, f_kslice(K + 1);
     for (int u = 0; u < U; ++u) {
         kslice[u] = (int32_t)sl_key.size();
-        const int64_t a = hks[u * C], cnt = hks[(u + 1) * C] - a;
-        const int64_t ranges = (cnt + kSliceCells - 1) / kSliceCells;
-        for (int64_t q = 1; q <= ranges; ++q) {
-            sl_start.push_back((int32_t)(a + cnt * q / ranges));
-            sl_key.push_back(u);
+        const int step = by_cluster ? 1 : C;
+        for (int k = u * C; k < (u + 1) * C; k += step) {
+            const int64_t a = hks[k], cnt = hks[k + step] - a;
+            const int64_t ranges = (cnt + kSliceCells - 1) / kSliceCells;
+            for (int64_t q = 1; q <= ranges; ++q) {
+                sl_start.push_back((int32_t)(a + cnt * q / ranges));
+                sl_key.push_back(u);
+            }
         }
     }
     kslice[U] = (int32_t)sl_key.size();
@@ -754,10 +772,14 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     double* rs = ws<double>(ctx, "grp_rs", (size_t)nrules * kRuleCap);
     double* rw = ws<double>(ctx, "grp_rw", (size_t)nrules * kRuleCap);
     int32_t* rm = ws<int32_t>(ctx, "grp_rm", nrules);
-    double* scr = ws<double>(ctx, "grp_scr", (size_t)6 * n);
+    double* scr = ws<double>(ctx, "grp_scr", (size_t)4 * n);
     double* rerr = ws<double>(ctx, "grp_rerr", nrules);
-    LAUNCH(launch_group_rules(permC, gsC, permF, gsF, U, nrules, dp.off, n, scr, rs, rw, rm, rerr,
-                              bad + 1, st));
+    // (MLE: the rules' sums in one order whatever the group sizes, as for the slices)
+    const bool one_block = overdispersion == DEVIL_OD_MLE;
+    LAUNCH(launch_group_rules(permC, gsC, U, dp.off, n, scr, rs, rw, rm, rerr, bad + 1, one_block, st));
+    if (C > 1)  // rules U.. : the (row, cluster) groups
+        LAUNCH(launch_group_rules(permF, gsF, K, dp.off, n, scr, rs + (size_t)U * kRuleCap,
+                                  rw + (size_t)U * kRuleCap, rm + U, rerr + U, bad + 1, one_block, st));
     dbg_mark(ctx, "g.rules");
     // CSR copy ordered by slice within each gene: 4-byte entries (index in
     // the slice, 16-bit count) or 8-byte ones for float counts
@@ -960,6 +982,14 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     g.rm = rm;
 }
 
+// the per-cell images where a per-cell engine will run: a design that is not
+// grouped, a clustered bread/meat that is not grouped by these clusters, and
+// the "new" dispersion
+void cells_if_needed(devil_ctx* ctx, DevProblem& dp, int n_clusters, int overdispersion) {
+    if (!dp.grp.active || (n_clusters > 0 && dp.grp.C != n_clusters) || overdispersion == DEVIL_OD_NEW)
+        prepare_cells(ctx, dp);
+}
+
 GrpGeom grp_geom(const DevProblem& dp) {
     const auto& gr = dp.grp;
     GrpGeom gg{};
@@ -1135,6 +1165,7 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
                  int nbound, const int32_t* act, const int32_t* n_act, int32_t* reset_next,
                  const PassBuffers& pb, const PassParamsAny& prm, int fine = 0,
                  const int32_t* n_heavy = nullptr, bool rowexp_fresh = false) {
+    if (plan.engine != ENGINE_GRP && !dp.Xrm) fail(ctx, DEVIL_ERR_ARG, "per-cell pass without the per-cell design");
     PassLaunch L;
     L.kind = kind;
     L.engine = plan.engine;
@@ -1875,7 +1906,7 @@ void fit_pipeline(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     dp.precision = o->precision;
     dbg_mark(ctx, "groups");
     LAUNCH(launch_theta0(dp.stats, dp.off, G, dp.n, o->has_init_overdispersion,
-                         o->init_overdispersion, fb.theta0, fb.k, st));
+                         o->init_overdispersion, ws<double>(ctx, "exp_off", dp.n), fb.theta0, fb.k, st));
     double* ginv = ws<double>(ctx, "ginv", (size_t)P * P);
     int32_t* err = ws<int32_t>(ctx, "qr_err", 1);
     if (!o->init_beta_rough) {
@@ -2115,7 +2146,8 @@ int devil_fit(devil_ctx* ctx, const devil_counts* counts, const double* X, int p
         dbg_mark(ctx, "design");
         compute_offsets(ctx, dp, opts->size_factors, opts->size_factor_values, nullptr, opts->offset);
         dbg_mark(ctx, "offsets");
-        build_groups(ctx, dp, cluster_ends, n_clusters, opts->form);
+        build_groups(ctx, dp, cluster_ends, n_clusters, opts->form, opts->overdispersion);
+        cells_if_needed(ctx, dp, n_clusters, opts->overdispersion);
         FitBuffers fb;
         alloc_fit_buffers(ctx, dp.G, p, res->theta_mom && opts->compute_theta_mom, n_clusters > 0, fb);
         fit_pipeline(ctx, dp, cluster_ends, n_clusters, opts, fb);
@@ -2197,7 +2229,8 @@ int devil_fit_device(devil_ctx* ctx, const devil_counts* counts_dev, const doubl
         dbg_mark(ctx, "design");
         compute_offsets(ctx, dp, opts->size_factors, nullptr, opts->size_factor_values, opts->offset);
         dbg_mark(ctx, "offsets");
-        build_groups(ctx, dp, cluster_ends_host, n_clusters, opts->form);
+        build_groups(ctx, dp, cluster_ends_host, n_clusters, opts->form, opts->overdispersion);
+        cells_if_needed(ctx, dp, n_clusters, opts->overdispersion);
         FitBuffers fb;
         alloc_fit_buffers(ctx, dp.G, p, r->theta_mom && opts->compute_theta_mom, n_clusters > 0, fb);
         // write straight into the caller's device buffers where given
@@ -2337,7 +2370,8 @@ int devil_estimate_dispersion(devil_ctx* ctx, const devil_counts* counts,
         upload_offsets(ctx, dp, offset_vector);
         double* th = ws<double>(ctx, "theta0", dp.G);
         float* k = ws<float>(ctx, "k", dp.G);
-        LAUNCH(launch_theta0(dp.stats, dp.off, dp.G, dp.n, 0, 0.0, th, k, ctx->stream));
+        LAUNCH(launch_theta0(dp.stats, dp.off, dp.G, dp.n, 0, 0.0, ws<double>(ctx, "exp_off", dp.n), th, k,
+                             ctx->stream));
         d2h(ctx, theta0, th, dp.G);
         CK(cudaStreamSynchronize(ctx->stream));
     });
@@ -2350,6 +2384,7 @@ int devil_init_beta(devil_ctx* ctx, const devil_counts* counts, const double* X,
         DevProblem dp;
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
+        prepare_cells(ctx, dp);
         upload_offsets(ctx, dp, offset_vector);
         double* ginv = ws<double>(ctx, "ginv", (size_t)p * p);
         int32_t* err = ws<int32_t>(ctx, "qr_err", 1);
@@ -2380,7 +2415,8 @@ int devil_beta_fit(devil_ctx* ctx, const devil_counts* counts, const double* X, 
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
         upload_offsets(ctx, dp, offset_vector);
-        build_groups(ctx, dp, nullptr, 0, form);
+        build_groups(ctx, dp, nullptr, 0, form, DEVIL_OD_NONE);
+        cells_if_needed(ctx, dp, 0, DEVIL_OD_NONE);
         const int64_t G = dp.G;
         double* b = ws<double>(ctx, "beta", (size_t)G * p);
         float* bf = ws<float>(ctx, "beta_f", (size_t)G * p);
@@ -2422,7 +2458,8 @@ int devil_estimate_mom_dispersion(devil_ctx* ctx, const devil_counts* counts, co
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
         upload_sf_as_offsets(ctx, dp, size_factors);
-        build_groups(ctx, dp, nullptr, 0, DEVIL_FORM_CHOSEN);
+        build_groups(ctx, dp, nullptr, 0, DEVIL_FORM_CHOSEN, DEVIL_OD_NONE);
+        cells_if_needed(ctx, dp, 0, DEVIL_OD_NONE);
         float* bf;
         double* bd;
         upload_beta(ctx, dp, beta, &bf, &bd);
@@ -2442,7 +2479,8 @@ int devil_fit_dispersion(devil_ctx* ctx, const devil_counts* counts, const doubl
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
         upload_offsets(ctx, dp, offset_vector);
-        build_groups(ctx, dp, nullptr, 0, DEVIL_FORM_CHOSEN);
+        build_groups(ctx, dp, nullptr, 0, DEVIL_FORM_CHOSEN, DEVIL_OD_MLE);
+        cells_if_needed(ctx, dp, 0, DEVIL_OD_NONE);
         float* bf;
         double* bd;
         upload_beta(ctx, dp, beta, &bf, &bd);
@@ -2469,6 +2507,7 @@ int devil_fit_overdispersion_new(devil_ctx* ctx, const devil_counts* counts, con
         DevProblem dp;
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
+        prepare_cells(ctx, dp);
         upload_offsets(ctx, dp, offset_vector);
         float* bf;
         double* bd;
@@ -2491,7 +2530,8 @@ int devil_compute_hessian(devil_ctx* ctx, const devil_counts* counts, const doub
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
         upload_sf_as_offsets(ctx, dp, size_factors);
-        build_groups(ctx, dp, nullptr, 0, DEVIL_FORM_CHOSEN);
+        build_groups(ctx, dp, nullptr, 0, DEVIL_FORM_CHOSEN, DEVIL_OD_NONE);
+        cells_if_needed(ctx, dp, 0, DEVIL_OD_NONE);
         float* bf;
         double* bd;
         upload_beta(ctx, dp, beta, &bf, &bd);
@@ -2515,7 +2555,8 @@ int devil_compute_clustered_meat(devil_ctx* ctx, const devil_counts* counts, con
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
         upload_sf_as_offsets(ctx, dp, size_factors);
-        build_groups(ctx, dp, cluster_ends, n_clusters, DEVIL_FORM_CHOSEN);
+        build_groups(ctx, dp, cluster_ends, n_clusters, DEVIL_FORM_CHOSEN, DEVIL_OD_NONE);
+        cells_if_needed(ctx, dp, n_clusters, DEVIL_OD_NONE);
         float* bf;
         double* bd;
         upload_beta(ctx, dp, beta, &bf, &bd);

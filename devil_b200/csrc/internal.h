@@ -286,10 +286,11 @@ cudaError_t launch_fine_keys(const int32_t* ucell, const int32_t* ends, int C, i
 cudaError_t launch_group_starts(const int32_t* ks, int64_t n, int K, int64_t* gstart,
                                 cudaStream_t st);
 cudaError_t launch_exp(const double* x, int64_t n, double* y, cudaStream_t st);
-cudaError_t launch_group_rules(const int32_t* permC, const int64_t* gsC, const int32_t* permF,
-                               const int64_t* gsF, int U, int nrules, const double* off, int64_t n,
+// the rules of the groups perm[gs[b]..gs[b+1]) (cells sorted by offset within
+// a group); scr: 4 n doubles
+cudaError_t launch_group_rules(const int32_t* perm, const int64_t* gs, int nrules, const double* off, int64_t n,
                                double* scr, double* rs, double* rw, int32_t* rm, double* rerr,
-                               int32_t* bad, cudaStream_t st);
+                               int32_t* bad, bool one_block, cudaStream_t st);
 cudaError_t launch_gather_keys(const int32_t* keys, const int32_t* cells, int64_t n, int32_t* out,
                                cudaStream_t st);
 int group_csr_segment(int64_t nnz, int64_t G, int K);  // entries per segment
@@ -335,12 +336,12 @@ cudaError_t launch_colstats(const int64_t* rowptr, const int32_t* col, const voi
 cudaError_t launch_sf_finalize(int method, int64_t G, int64_t n, const double* colsum,
                                const double* collog, const int32_t* colcnt,
                                const int32_t* colmin_bits, double offset, double* sf,
-                               double* off, float* off_f, int32_t* err, cudaStream_t st);
+                               double* off, float* off_f, double* gm, int32_t* err, cudaStream_t st);
 cudaError_t launch_sf_given(const double* sf_in, int64_t n, double offset, int use_sf, double* sf,
                             double* off, float* off_f, cudaStream_t st);
 cudaError_t launch_theta0(const double* stats, const double* off, int64_t G, int64_t n,
-                          int has_init, double init_value, double* theta0, float* k,
-                          cudaStream_t st);
+                          int has_init, double init_value, double* eoff, double* theta0, float* k,
+                          cudaStream_t st);  // eoff: n doubles of scratch
 int xtx_blocks(int64_t n);  // partial-sum blocks launch_xtx_inverse needs
 cudaError_t launch_xtx_inverse(const double* Xcm, int64_t n, int P, double* part, double* ginv,
                                int32_t* err, cudaStream_t st);

@@ -23,11 +23,14 @@
 // (for one-hot rows: a handful per group), instead of O(cells x p^2).  Partial sums land in the layout of the other engines
 // (FP64, one segment, or one per cluster for the sandwich), so the
 // finalize kernels are shared.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <type_traits>
 
 #include "internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace devil {
 
@@ -126,30 +129,36 @@ __global__ void exp_kernel(const double* x, int64_t n, double* y) {
 // ---------------------------------------------------------------------
 // Gauss rules of the groups' offset distributions
 // ---------------------------------------------------------------------
-constexpr int kRuleNT = 256;
+constexpr int kRuleNT = 512;   // threads of a rule's blocks
+constexpr int kRuleNT1 = 256;  // of its one block, where the sums keep one order
 
-// block-wide sum; every thread gets the same value (same association)
-DEV double block_sum(double v, double* red) {
-    v = warp_sum(v);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncthreads();
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    double r = l < nw ? red[l] : 0.0;
-    return warp_sum(r);
-}
-DEV double block_min(double v, double* red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncthreads();
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    double r = l < nw ? red[l] : INFINITY;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) r = fmin(r, __shfl_xor_sync(0xffffffffu, r, o));
-    return r;
-}
+// The blocks of one rule: a cluster of up to eight, whose threads split the
+// group's cells.  sum() gives every thread the same value (same association);
+// two slots in turn keep a fast block from overwriting a sum that a slow one
+// still reads.
+struct RuleBlocks {
+    cg::cluster_group cl;
+    int rank, nb, t, nt;
+    double* red;   // [32]
+    double* part;  // [2]
+    int slot;
+    DEV double sum(double v) {
+        v = warp_sum(v);
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+        __syncthreads();
+        if (l == 0) red[w] = v;
+        __syncthreads();
+        double r = l < nw ? red[l] : 0.0;
+        r = warp_sum(r);
+        if (nb == 1) return r;
+        if (threadIdx.x == 0) part[slot] = r;
+        cl.sync();
+        r = 0.0;
+        for (int k = 0; k < nb; ++k) r += *cl.map_shared_rank(part + slot, k);
+        slot ^= 1;
+        return r;
+    }
+};
 
 // number of eigenvalues below x of the Jacobi matrix with diagonal al[0..m)
 // and squared off-diagonal be[1..m) (Sturm sequence of the LDL^T pivots)
@@ -164,7 +173,7 @@ DEV int jacobi_count_below(const double* al, const double* be, int m, double x) 
     return c;
 }
 
-// Gauss rule of one bin of sorted offsets s[perm[c0..c1)] (more than
+// Gauss rule of one bin of sorted offsets s[c0..c1) (more than
 // kBinNodes cells, a spread above 1e-13) with m <= kBinNodes nodes, written
 // to os/ow.  In t = (s - c)/h the monic orthogonal polynomials of the bin's
 // measure are run over its cells (discretised Stieltjes procedure, stable
@@ -172,23 +181,24 @@ DEV int jacobi_count_below(const double* al, const double* be, int m, double x) 
 // (bisection on Sturm counts), the weights the Christoffel numbers scaled
 // to the bin's cell count.  The recurrence stops early when pi_{k+1}
 // vanishes on the support (at most k+1 distinct offsets: the rule is then
-// exact).  Returns m (same value in every thread).
-DEV int bin_rule(const int32_t* perm, const double* off, int64_t c0, int64_t c1, double* tt,
-                 double* p0, double* p1, double* red, double* al, double* be, double* nk,
+// exact).  Returns m (same value in every thread of the cluster; block 0
+// writes the rule).
+DEV int bin_rule(RuleBlocks& rb, const double* soff, int64_t c0, int64_t c1, double* tt,
+                 double* p0, double* p1, double* al, double* be, double* nk,
                  double* wsum, double* os, double* ow) {
-    const int t = threadIdx.x, nt = blockDim.x;
+    const int t = threadIdx.x;
     const double cnt = (double)(c1 - c0);
-    const double bmin = off[perm[c0]], bmax = off[perm[c1 - 1]];
+    const double bmin = soff[c0], bmax = soff[c1 - 1];
     const double c = 0.5 * (bmax + bmin), h = 0.5 * (bmax - bmin);
     double st = 0.0;
-    for (int64_t i = c0 + t; i < c1; i += nt) {
-        const double x = (off[perm[i]] - c) / h;
+    for (int64_t i = c0 + rb.t; i < c1; i += rb.nt) {
+        const double x = (soff[i] - c) / h;
         tt[i] = x;
         p0[i] = 1.0;
         p1[i] = 0.0;
         st += x;
     }
-    st = block_sum(st, red);
+    st = rb.sum(st);
     if (t == 0) {
         al[0] = st / cnt;
         be[0] = 0.0;
@@ -199,7 +209,7 @@ DEV int bin_rule(const int32_t* perm, const double* off, int64_t c0, int64_t c1,
     for (int k = 0; k + 1 < kBinNodes; ++k) {
         const double a = al[k], bb = be[k];
         double sN = 0.0, sT = 0.0, sS = 0.0;
-        for (int64_t i = c0 + t; i < c1; i += nt) {
+        for (int64_t i = c0 + rb.t; i < c1; i += rb.nt) {
             const double x = tt[i], pk = p0[i], pm = p1[i];
             const double pn = (x - a) * pk - bb * pm;
             const double sc = fabs(x - a) * fabs(pk) + bb * fabs(pm);
@@ -209,9 +219,9 @@ DEV int bin_rule(const int32_t* perm, const double* off, int64_t c0, int64_t c1,
             sT += x * pn * pn;
             sS += sc * sc;
         }
-        sN = block_sum(sN, red);
-        sT = block_sum(sT, red);
-        sS = block_sum(sS, red);
+        sN = rb.sum(sN);
+        sT = rb.sum(sT);
+        sS = rb.sum(sS);
         if (!(sN > 1e-26 * sS)) {  // pi_{k+1} is rounding noise on the support
             m = k + 1;
             break;
@@ -249,7 +259,7 @@ DEV int bin_rule(const int32_t* perm, const double* off, int64_t c0, int64_t c1,
     if (t < 32) {
         double v = t < m ? wsum[t] : 0.0;
         v = warp_sum(v);
-        if (t < m) {
+        if (t < m && rb.rank == 0) {
             os[t] = c + h * xj;
             ow[t] = wj * (cnt / v);  // weights sum to the bin's cell count
         }
@@ -258,56 +268,55 @@ DEV int bin_rule(const int32_t* perm, const double* off, int64_t c0, int64_t c1,
     return m;
 }
 
-// first position in [lo, hi) of the sorted offsets s[perm[.]] with s >= v
-DEV int64_t lower_bound_off(const int32_t* perm, const double* off, int64_t lo, int64_t hi, double v) {
+// first position in [lo, hi) of the sorted offsets s with s >= v
+DEV int64_t lower_bound_off(const double* soff, int64_t lo, int64_t hi, double v) {
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
-        if (off[perm[mid]] < v) lo = mid + 1; else hi = mid;
+        if (soff[mid] < v) lo = mid + 1; else hi = mid;
     }
     return lo;
 }
 
-// Block per rule.  Rule b < U: coarse group b, cells permC[gsC[b]..gsC[b+1])
-// sorted by offset; rule U + k: fine group k (row, cluster), cells
-// permF[gsF[k]..gsF[k+1]).  The group's offsets are cut into bins of width
-// kBinWidth; a bin of at most kBinNodes cells contributes its cells as
-// nodes (weight 1), a bin of one offset (to 1e-13) one node at its mean,
-// any other bin a kBinNodes-point Gauss rule (bin_rule).  With bins of
-// width 2 the dense terms of the passes, analytic within pi of the real
-// s axis, are integrated to ~1e-15.  The rule is checked on
-// sum_i 1/(1 + exp(s_i - z)) for z at both ends and the middle of the
-// group's range; rerr[b] is the worst relative error and a value above
+// A block or a cluster of blocks per rule.  Rule b of this launch: group b of
+// `perm` (cells perm[gs[b]..gs[b+1]), sorted by offset; soff: their offsets).
+// The group's offsets are cut into bins of width kBinWidth; a bin of at most
+// kBinNodes cells contributes its cells as nodes (weight 1), a bin of one
+// offset (to 1e-13) one node at its mean, any other bin a kBinNodes-point
+// Gauss rule (bin_rule).  With bins of width 2 the dense terms of the passes,
+// analytic within pi of the real s axis, are integrated to ~1e-15.  The rule
+// is checked on sum_i 1/(1 + exp(s_i - z)) for z at both ends and the middle
+// of the group's range; rerr[b] is the worst relative error and a value above
 // 1e-11 (or more than kMaxBins bins) sets *bad.
+// A few large groups (two conditions of half a million cells) leave one block
+// per rule with dozens of passes over the group to itself: 4.14 ms; clusters
+// of eight and the gathered offsets take it to 0.18 ms.
 __global__ void __launch_bounds__(kRuleNT) group_rules_kernel(
-    const int32_t* permC, const int64_t* gsC, const int32_t* permF, const int64_t* gsF, int U,
-    const double* off, int64_t n, double* scr, double* rs, double* rw, int32_t* rm, double* rerr,
-    int32_t* bad) {
-    __shared__ double red[32];
+    const double* soff, const int64_t* gs, int blocks, int64_t n, double* scr, double* rs, double* rw,
+    int32_t* rm, double* rerr, int32_t* bad) {
+    __shared__ double red[32], part[2];
     __shared__ double al[kBinNodes + 1], be[kBinNodes + 1], nk[kBinNodes + 1];
     __shared__ double wsum[32];
     __shared__ int64_t rng[2];
-    const int b = blockIdx.x, t = threadIdx.x, nt = blockDim.x;
-    const bool coarse = b < U;
-    const int32_t* perm = coarse ? permC : permF;
-    const int64_t b0 = coarse ? gsC[b] : gsF[b - U];
-    const int64_t b1 = coarse ? gsC[b + 1] : gsF[b - U + 1];
-    const int64_t base = coarse ? 0 : n;  // scratch of coarse and fine rules
-    double* tt = scr + base;
-    double* p0 = scr + 2 * n + base;
-    double* p1 = scr + 4 * n + base;
+    const int b = blockIdx.x / blocks, t = threadIdx.x;
+    const int rank = blockIdx.x % blocks;
+    RuleBlocks rb{cg::this_cluster(), rank, blocks, rank * (int)blockDim.x + t, blocks * (int)blockDim.x, red, part, 0};
+    const int64_t b0 = gs[b], b1 = gs[b + 1];
+    double* tt = scr;
+    double* p0 = scr + n;
+    double* p1 = scr + 2 * n;
     double* os = rs + (int64_t)b * kRuleCap;
     double* ow = rw + (int64_t)b * kRuleCap;
     if (b1 <= b0) {
-        if (t == 0) {
+        if (rb.t == 0) {
             rm[b] = 0;
             rerr[b] = 0.0;
         }
         return;
     }
-    const double smin = off[perm[b0]], smax = off[perm[b1 - 1]];
+    const double smin = soff[b0], smax = soff[b1 - 1];
     const double span = (smax - smin) / kBinWidth;
     if (!(span < (double)kMaxBins)) {  // offsets too spread (or not finite)
-        if (t == 0) {
+        if (rb.t == 0) {
             rm[b] = 0;
             rerr[b] = INFINITY;
             atomicExch(bad, 1);
@@ -318,8 +327,8 @@ __global__ void __launch_bounds__(kRuleNT) group_rules_kernel(
     int nodes = 0;
     for (int j = 0; j < nb; ++j) {
         if (t == 0) {
-            rng[0] = j == 0 ? b0 : lower_bound_off(perm, off, b0, b1, smin + j * kBinWidth);
-            rng[1] = j == nb - 1 ? b1 : lower_bound_off(perm, off, b0, b1, smin + (j + 1) * kBinWidth);
+            rng[0] = j == 0 ? b0 : lower_bound_off(soff, b0, b1, smin + j * kBinWidth);
+            rng[1] = j == nb - 1 ? b1 : lower_bound_off(soff, b0, b1, smin + (j + 1) * kBinWidth);
         }
         __syncthreads();
         const int64_t c0 = rng[0], c1 = rng[1];
@@ -327,47 +336,48 @@ __global__ void __launch_bounds__(kRuleNT) group_rules_kernel(
         const int64_t cnt = c1 - c0;
         if (cnt <= 0) continue;
         if (cnt <= kBinNodes) {
-            if (t < cnt) {
-                os[nodes + t] = off[perm[c0 + t]];
+            if (rb.t < cnt) {
+                os[nodes + t] = soff[c0 + t];
                 ow[nodes + t] = 1.0;
             }
             nodes += (int)cnt;
             continue;
         }
-        const double bmin = off[perm[c0]], bmax = off[perm[c1 - 1]];
+        const double bmin = soff[c0], bmax = soff[c1 - 1];
         if (!(bmax - bmin > 1e-13 * fmax(1.0, fabs(bmax)))) {
             double sm = 0.0;
-            for (int64_t i = c0 + t; i < c1; i += nt) sm += off[perm[i]];
-            sm = block_sum(sm, red);
-            if (t == 0) {
+            for (int64_t i = c0 + rb.t; i < c1; i += rb.nt) sm += soff[i];
+            sm = rb.sum(sm);
+            if (rb.t == 0) {
                 os[nodes] = sm / (double)cnt;
                 ow[nodes] = (double)cnt;
             }
             nodes += 1;
             continue;
         }
-        nodes += bin_rule(perm, off, c0, c1, tt, p0, p1, red, al, be, nk, wsum, os + nodes,
-                          ow + nodes);
+        nodes += bin_rule(rb, soff, c0, c1, tt, p0, p1, al, be, nk, wsum, os + nodes, ow + nodes);
     }
-    if (t == 0) rm[b] = nodes;
-    __syncthreads();
+    if (rb.t == 0) rm[b] = nodes;
+    __syncthreads();  // (block 0 reads its own writes of the rule below)
     // check the rule against exact sums of three logistic test functions
     const double mid = 0.5 * (smin + smax);
     double worst = 0.0;
     for (int z = 0; z < 3; ++z) {
         const double zc = z == 0 ? smin : (z == 1 ? mid : smax);
         double ex = 0.0, ap = 0.0;
-        for (int64_t i = b0 + t; i < b1; i += nt) ex += 1.0 / (1.0 + exp(off[perm[i]] - zc));
-        for (int i = t; i < nodes; i += nt) ap += ow[i] / (1.0 + exp(os[i] - zc));
-        ex = block_sum(ex, red);
-        ap = block_sum(ap, red);
+        for (int64_t i = b0 + rb.t; i < b1; i += rb.nt) ex += 1.0 / (1.0 + exp(soff[i] - zc));
+        if (rank == 0)
+            for (int i = t; i < nodes; i += (int)blockDim.x) ap += ow[i] / (1.0 + exp(os[i] - zc));
+        ex = rb.sum(ex);
+        ap = rb.sum(ap);
         const double e = fabs(ap - ex) / ex;
         worst = e > worst ? e : (e == e ? worst : e);  // NaN sticks
     }
-    if (t == 0) {
+    if (rb.t == 0) {
         rerr[b] = worst;
         if (!(worst <= 1e-11)) atomicExch(bad, 1);
     }
+    if (blocks > 1) rb.cl.sync();  // no block leaves while another reads its sums
 }
 
 // ---------------------------------------------------------------------
@@ -1505,13 +1515,32 @@ cudaError_t launch_exp(const double* x, int64_t n, double* y, cudaStream_t st) {
     exp_kernel<<<nblk(n, 256), 256, 0, st>>>(x, n, y);
     return cudaGetLastError();
 }
-cudaError_t launch_group_rules(const int32_t* permC, const int64_t* gsC, const int32_t* permF,
-                               const int64_t* gsF, int U, int nrules, const double* off, int64_t n,
+__global__ void gather_d_kernel(const double* x, const int32_t* idx, int64_t n, double* out) {
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = x[idx[i]];
+}
+cudaError_t launch_group_rules(const int32_t* perm, const int64_t* gs, int nrules, const double* off, int64_t n,
                                double* scr, double* rs, double* rw, int32_t* rm, double* rerr,
-                               int32_t* bad, cudaStream_t st) {
-    group_rules_kernel<<<(unsigned)nrules, kRuleNT, 0, st>>>(permC, gsC, permF, gsF, U, off, n, scr,
-                                                             rs, rw, rm, rerr, bad);
-    return cudaGetLastError();
+                               int32_t* bad, bool one_block, cudaStream_t st) {
+    if (nrules <= 0) return cudaSuccess;
+    double* soff = scr + 3 * n;
+    gather_d_kernel<<<nblk(n, 256), 256, 0, st>>>(off, perm, n, soff);
+    // blocks per rule by the mean cells of a group: 16,384 cells are 32 rounds of
+    // one block (62 rules of 16,000 cells: 434 us with one block, 285 us with two)
+    const int64_t mean = n / nrules;
+    const int blocks = one_block ? 1 : (mean >= 65536 ? 8 : (mean >= 16384 ? 4 : (mean >= 8192 ? 2 : 1)));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(nrules * blocks));
+    cfg.blockDim = dim3(one_block ? kRuleNT1 : kRuleNT);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, group_rules_kernel, (const double*)soff, gs, blocks, n, scr, rs, rw, rm, rerr, bad);
 }
 int group_csr_segment(int64_t nnz, int64_t G, int K) {
     int S = 2048;  // entries per segment; the count table stays below 2^27 entries

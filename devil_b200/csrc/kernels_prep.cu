@@ -580,33 +580,57 @@ cudaError_t launch_colstats(const int64_t* rowptr, const int32_t* col, const voi
     return cudaGetLastError();
 }
 
-// size factors from the column statistics; one block.
+// sum of f over c = t, t + T, ... (T threads), 16 loads in flight per thread
+// and added in that order
+template <class F>
+DEV double strided_sum(int64_t n, F&& at) {
+    constexpr int U = 16;
+    const int64_t T = blockDim.x;
+    double acc = 0.0;
+    for (int64_t c = threadIdx.x; c < n; c += T * U) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = c + T * u < n ? at(c + T * u) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c + T * u < n) acc += v[u];
+    }
+    return acc;
+}
+
+// size factors from the column statistics.
 // method 1 = normed_sum (R/size_factors.R:75-88), 2 = psinorm (:100-117).
-__global__ void sf_finalize_kernel(int method, int64_t G, int64_t n, const double* colsum,
-                                   const double* collog, const int32_t* colcnt,
-                                   const int32_t* colmin_bits, double offset, double* sf,
-                                   double* off, float* off_f, int32_t* err) {
-    __shared__ double red[32];
-    __shared__ double red2[32];
-    __shared__ double gm_s;
-    double acc = 0.0, cntv = 0.0;
-    int zero = 0;
-    for (int64_t c = threadIdx.x; c < n; c += blockDim.x) {
+// The logarithms on every SM, then one block for their sum (in a fixed order),
+// then the division and the offsets on every SM: one block for all of it took
+// 1.29 ms at a million cells, the three take 0.25 ms.
+__global__ void sf_log_kernel(int method, int64_t G, int64_t n, const double* colsum, const double* collog,
+                              const int32_t* colcnt, const int32_t* colmin_bits, double* sf, double* lg,
+                              int32_t* err) {
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
+         c += (int64_t)gridDim.x * blockDim.x) {
         double v;
         if (G <= 1) {
             v = 1.0;
         } else if (method == 1) {
             v = colsum[c];
-            if (v == 0.0) zero = 1;
+            if (v == 0.0) *err = 1;
         } else {
             double m = colcnt[c] < G ? 0.0 : (double)__int_as_float(colmin_bits[c]);
             v = collog[c] / (double)G - m;
         }
         sf[c] = v;
-        double l = log(v);
-        if (!isnan(l)) { acc += l; cntv += 1.0; }
+        lg[c] = log(v);
     }
-    zero = __syncthreads_or(zero);
+}
+__global__ void __launch_bounds__(1024) sf_mean_kernel(int64_t G, int64_t n, const double* lg, double* gm) {
+    __shared__ double red[32], red2[32];
+    double cntv = 0.0;
+    double acc = strided_sum(n, [&](int64_t c) {
+        const double l = lg[c];
+        const bool ok = !isnan(l);
+        cntv += ok ? 1.0 : 0.0;
+        return ok ? l : 0.0;
+    });
     acc = warp_sum(acc);
     cntv = warp_sum(cntv);
     if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = acc; red2[threadIdx.x >> 5] = cntv; }
@@ -614,12 +638,14 @@ __global__ void sf_finalize_kernel(int method, int64_t G, int64_t n, const doubl
     if (threadIdx.x == 0) {
         double s = 0.0, k = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { s += red[w]; k += red2[w]; }
-        gm_s = (G <= 1) ? 1.0 : exp(s / k);
-        if (err) *err = (method == 1 && zero && G > 1) ? 1 : 0;
+        *gm = (G <= 1) ? 1.0 : exp(s / k);
     }
-    __syncthreads();
-    const double gm = gm_s;
-    for (int64_t c = threadIdx.x; c < n; c += blockDim.x) {
+}
+__global__ void sf_scale_kernel(int64_t G, int64_t n, const double* gm_p, double offset, double* sf, double* off,
+                                float* off_f) {
+    const double gm = *gm_p;
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
+         c += (int64_t)gridDim.x * blockDim.x) {
         double v = (G <= 1) ? 1.0 : sf[c] / gm;
         sf[c] = v;
         double o = offset + log(v);
@@ -630,9 +656,13 @@ __global__ void sf_finalize_kernel(int method, int64_t G, int64_t n, const doubl
 cudaError_t launch_sf_finalize(int method, int64_t G, int64_t n, const double* colsum,
                                const double* collog, const int32_t* colcnt,
                                const int32_t* colmin_bits, double offset, double* sf,
-                               double* off, float* off_f, int32_t* err, cudaStream_t st) {
-    sf_finalize_kernel<<<1, 1024, 0, st>>>(method, G, n, colsum, collog, colcnt, colmin_bits,
-                                           offset, sf, off, off_f, err);
+                               double* off, float* off_f, double* gm, int32_t* err, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int32_t), st);
+    if (e != cudaSuccess) return e;
+    const unsigned b = (unsigned)std::min<int64_t>(nblk(n, 256), 148 * 8);
+    sf_log_kernel<<<b, 256, 0, st>>>(method, G, n, colsum, collog, colcnt, colmin_bits, sf, off, err);
+    sf_mean_kernel<<<1, 1024, 0, st>>>(G, n, off, gm);
+    sf_scale_kernel<<<b, 256, 0, st>>>(G, n, gm, offset, sf, off, off_f);
     return cudaGetLastError();
 }
 
@@ -662,12 +692,18 @@ cudaError_t launch_sf_given(const double* sf_in, int64_t n, double offset, int u
 // (R/overdispersion.R:129-135); k = 1/theta_0 as the float beta_fit keeps
 // (src/beta.cpp:25-28: theta_0 arrives as float, 1.0/k stored as float).
 // ------------------------------------------------------------------
-__global__ void theta0_kernel(const double* stats, const double* off, int64_t G, int64_t n,
-                              int has_init, double init_value, double* theta0, float* k) {
+// eoff = exp(off), evaluated on every SM beforehand (this kernel's one block
+// took 0.53 ms for a million cells, the two take 0.14 ms)
+__global__ void exp_off_kernel(const double* off, int64_t n, double* eoff) {
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
+         c += (int64_t)gridDim.x * blockDim.x)
+        eoff[c] = exp(off[c]);
+}
+__global__ void __launch_bounds__(1024) theta0_kernel(const double* stats, const double* eoff, int64_t G, int64_t n,
+                                                      int has_init, double init_value, double* theta0, float* k) {
     __shared__ double red[32];
     __shared__ double moi_s;
-    double acc = 0.0;
-    for (int64_t c = threadIdx.x; c < n; c += blockDim.x) acc += exp(off[c]);
+    double acc = strided_sum(n, [&](int64_t c) { return eoff[c]; });
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
@@ -693,9 +729,11 @@ __global__ void theta0_kernel(const double* stats, const double* off, int64_t G,
     }
 }
 cudaError_t launch_theta0(const double* stats, const double* off, int64_t G, int64_t n,
-                          int has_init, double init_value, double* theta0, float* k,
+                          int has_init, double init_value, double* eoff, double* theta0, float* k,
                           cudaStream_t st) {
-    theta0_kernel<<<1, 1024, 0, st>>>(stats, off, G, n, has_init, init_value, theta0, k);
+    if (has_init) n = 0;  // theta_0 is given: no mean of exp(off)
+    if (n > 0) exp_off_kernel<<<(unsigned)std::min<int64_t>(nblk(n, 256), 148 * 8), 256, 0, st>>>(off, n, eoff);
+    theta0_kernel<<<1, 1024, 0, st>>>(stats, eoff, G, n, has_init, init_value, theta0, k);
     return cudaGetLastError();
 }
 
@@ -703,8 +741,10 @@ cudaError_t launch_theta0(const double* stats, const double* off, int64_t G, int
 // (X'X)^-1 in FP64 (one block): the least-squares solve of init_beta
 // ------------------------------------------------------------------
 // partial X'X over the cells of one block (kXtxCells cells, staged in
-// shared memory 256 at a time, row stride P+1); thread t owns packed
-// pairs t, t + 256, ...
+// shared memory 256 at a time, row stride P+1); thread t of block y owns the
+// packed pair 256 y + t (up to three blocks share a range of cells: one block
+// whose threads owned three pairs each took 0.93 ms at p = 32 and a million
+// cells, these take 0.65 ms)
 constexpr int kXtxCells = 8192;
 constexpr int kXtxStage = 256;
 __global__ void __launch_bounds__(256) xtx_partial_kernel(const double* Xcm, int64_t n, int P,
@@ -714,16 +754,11 @@ __global__ void __launch_bounds__(256) xtx_partial_kernel(const double* Xcm, int
     const int RS = P + 1;
     const int64_t c0 = (int64_t)blockIdx.x * kXtxCells;
     const int64_t c1 = c0 + kXtxCells < n ? c0 + kXtxCells : n;
-    double acc[3] = {0.0, 0.0, 0.0};  // NP <= 528 = 256 * 3 (rounded up)
-    int pi[3], pj[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int q = threadIdx.x + k * 256;
-        int j = 0;
-        while ((j + 1) * (j + 2) / 2 <= q) ++j;
-        pi[k] = q < NP ? q - j * (j + 1) / 2 : 0;
-        pj[k] = q < NP ? j : 0;
-    }
+    const int q = blockIdx.y * 256 + threadIdx.x;
+    int j = 0;
+    while ((j + 1) * (j + 2) / 2 <= q) ++j;
+    const int pi = q < NP ? q - j * (j + 1) / 2 : 0, pj = q < NP ? j : 0;
+    double acc = 0.0;
     for (int64_t cb = c0; cb < c1; cb += kXtxStage) {
         const int nc = (int)(c1 - cb < kXtxStage ? c1 - cb : kXtxStage);
         __syncthreads();
@@ -732,30 +767,28 @@ __global__ void __launch_bounds__(256) xtx_partial_kernel(const double* Xcm, int
             xs[c * RS + col] = Xcm[(int64_t)col * n + cb + c];
         }
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            if (threadIdx.x + k * 256 >= NP) break;
-            double s = 0.0;
-            for (int c = 0; c < nc; ++c) s = fma(xs[c * RS + pi[k]], xs[c * RS + pj[k]], s);
-            acc[k] += s;
-        }
+        if (q >= NP) continue;
+        double s = 0.0;
+        for (int c = 0; c < nc; ++c) s = fma(xs[c * RS + pi], xs[c * RS + pj], s);
+        acc += s;
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int q = threadIdx.x + k * 256;
-        if (q < NP) part[(int64_t)blockIdx.x * NP + q] = acc[k];
-    }
+    if (q < NP) part[(int64_t)blockIdx.x * NP + q] = acc;
 }
 
-// sum the partials in block order (deterministic), then invert with LU;
+// sum the partials in block order (deterministic), then invert by LU with
+// partial pivoting: the row updates of a column over all threads, a thread per
+// column of the inverse (one thread for everything took 0.97 ms at p = 32, this
+// takes 0.13 ms);
 // rank check on the pivots relative to the largest diagonal
 __global__ void xtx_finish_kernel(const double* part, int nb, int P, double* ginv, int32_t* err) {
     extern __shared__ double sh[];
     double* Gm = sh;         // P*P
     double* W = sh + P * P;  // P*P
     int* piv = reinterpret_cast<int*>(W + P * P);
+    __shared__ int ok_s;
+    const int t = threadIdx.x, nt = blockDim.x;
     const int NP = P * (P + 1) / 2;
-    for (int q = threadIdx.x; q < NP; q += blockDim.x) {
+    for (int q = t; q < NP; q += nt) {
         int j = 0;
         while ((j + 1) * (j + 2) / 2 <= q) ++j;
         const int i = q - j * (j + 1) / 2;
@@ -765,16 +798,50 @@ __global__ void xtx_finish_kernel(const double* part, int nb, int P, double* gin
         Gm[i * P + j] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double dmax = 0.0;
-        for (int i = 0; i < P; ++i) dmax = fmax(dmax, fabs(Gm[i * P + i]));
-        bool ok = lu_factor(P, Gm, piv);
-        for (int i = 0; i < P; ++i)
-            if (!(fabs(Gm[i * P + i]) > 1e-12 * dmax)) ok = false;
-        if (ok) lu_inverse(P, Gm, piv, W);
-        for (int i = 0; i < P * P; ++i) ginv[i] = ok ? W[i] : NAN;
-        *err = ok ? 0 : 1;
+    double dmax = 0.0;
+    for (int i = 0; i < P; ++i) dmax = fmax(dmax, fabs(Gm[i * P + i]));
+    if (t == 0) ok_s = 1;
+    __syncthreads();
+    for (int k = 0; k < P; ++k) {
+        int mx = k;  // (every thread finds the same pivot)
+        double mv = fabs(Gm[k * P + k]);
+        for (int i = k + 1; i < P; ++i) {
+            const double v = fabs(Gm[k * P + i]);
+            if (v > mv) { mv = v; mx = i; }
+        }
+        __syncthreads();
+        if (t == 0) piv[k] = mx;
+        if (mx != k && t < P) {
+            const double x = Gm[t * P + k];
+            Gm[t * P + k] = Gm[t * P + mx];
+            Gm[t * P + mx] = x;
+        }
+        __syncthreads();
+        const double d = Gm[k * P + k];
+        if (t == 0 && (!(d != 0.0) || !isfinite(d))) ok_s = 0;
+        const double rd = 1.0 / d;
+        for (int i = k + 1 + t; i < P; i += nt) Gm[k * P + i] *= rd;
+        __syncthreads();
+        const int r = P - k - 1;
+        for (int q = t; q < r * r; q += nt) {
+            const int j = k + 1 + q / r, i = k + 1 + q % r;
+            Gm[j * P + i] -= Gm[k * P + i] * Gm[j * P + k];
+        }
+        __syncthreads();
     }
+    if (t == 0)
+        for (int i = 0; i < P; ++i)
+            if (!(fabs(Gm[i * P + i]) > 1e-12 * dmax)) ok_s = 0;
+    __syncthreads();
+    const bool ok = ok_s != 0;
+    if (ok && t < P) {
+        double* x = W + t * P;
+        for (int i = 0; i < P; ++i) x[i] = i == t ? 1.0 : 0.0;
+        lu_solve(P, Gm, piv, x);
+    }
+    __syncthreads();
+    for (int i = t; i < P * P; i += nt) ginv[i] = ok ? W[i] : NAN;
+    if (t == 0) *err = ok ? 0 : 1;
 }
 
 int xtx_blocks(int64_t n) { return (int)((n + kXtxCells - 1) / kXtxCells); }
@@ -787,12 +854,11 @@ cudaError_t launch_xtx_inverse(const double* Xcm, int64_t n, int P, double* part
     const size_t sm1 = (size_t)kXtxStage * (P + 1) * sizeof(double);
     cudaError_t e = raise_dyn_smem(xtx_partial_kernel, sm1);
     if (e != cudaSuccess) return e;
-    xtx_partial_kernel<<<nb, 256, sm1, st>>>(Xcm, n, P, part);
+    xtx_partial_kernel<<<dim3(nb, (P * (P + 1) / 2 + 255) / 256), 256, sm1, st>>>(Xcm, n, P, part);
     const size_t sm2 = (size_t)2 * P * P * 8 + (size_t)P * 4 + 16;
     xtx_finish_kernel<<<1, 256, sm2, st>>>(part, nb, P, ginv, err);
     return cudaGetLastError();
 }
-
 // beta_0 (warp per gene).  QR least squares of log1p(y / exp(off)) on X:
 // the solution equals (X'X)^-1 X' z; z is zero wherever y is zero, so
 // X' z is a sum over the nonzero entries of the row.  Rough init:
