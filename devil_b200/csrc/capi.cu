@@ -68,6 +68,7 @@ int pass_blocks_per_sm(PassKind kind, Engine engine, int P, int GT, int val_u16,
     else if (engine == ENGINE_GEN) e = launch_gen_pass(L);
     else if (engine == ENGINE_TC) e = launch_tc_pass(L, nullptr);
     else if (engine == ENGINE_TCW) e = launch_tcw_pass(L, TcwGeom{});
+    else if (engine == ENGINE_C64) e = launch_cell64_pass(L);
     if (e != cudaSuccess || occ < 1) {
         cudaGetLastError();  // a failed query leaves no sticky error; use one block per SM
         occ = 1;
@@ -1073,6 +1074,8 @@ PassPlan plan_engine(PassKind k, const DevProblem& dp, int form, bool allow_tcw 
     if (dp.grp.active) return {ENGINE_GRP, 1};
     if (k == PASS_IRLS && allow_tcw && tcw_wanted(dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
     if (k == PASS_MLE && allow_tcw && tcw_mle_wanted(dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
+    // bread/meat above the register engine's p: FP64 matrix tiles
+    if (P > reg_max_p() && cell64_supported(k, P, dp.xs)) return {ENGINE_C64, cell64_tile_genes()};
     const bool tc = tc_enabled(k) ||
                     (dp.precision == DEVIL_PREC_TC_TF32 && (k == PASS_IRLS || k == PASS_MLE));
     if (P <= tc_max_p() && tc) return {ENGINE_TC, tc_tile_genes(k)};
@@ -1164,7 +1167,7 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
                  int nseg, int tiles, const int32_t* bound, const int64_t* segptr,
                  int nbound, const int32_t* act, const int32_t* n_act, int32_t* reset_next,
                  const PassBuffers& pb, const PassParamsAny& prm, int fine = 0,
-                 const int32_t* n_heavy = nullptr, bool rowexp_fresh = false) {
+                 const int32_t* n_heavy = nullptr, bool rowexp_fresh = false, bool want_vec = true) {
     if (plan.engine != ENGINE_GRP && !dp.Xrm) fail(ctx, DEVIL_ERR_ARG, "per-cell pass without the per-cell design");
     PassLaunch L;
     L.kind = kind;
@@ -1199,7 +1202,8 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
     L.stream = ctx->stream;
     L.plain = plan.plain;
     size_t e0 = ctx->profiling ? prof_event(ctx) : 0;
-    ctx->last_engine[kind] = (int)plan.engine;
+    // (the FP64 matrix engine is the shared-memory tiles' engine to callers)
+    ctx->last_engine[kind] = (int)(plan.engine == ENGINE_C64 ? ENGINE_GEN : plan.engine);
     if (plan.engine == ENGINE_GRP) {
         GrpGeom gg = grp_geom(dp);
         gg.fine = fine;
@@ -1251,6 +1255,12 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
             dp.tcw_ready = true;
         }
         LAUNCH(launch_tcw_pass(L, dp.tcw));
+    } else if (plan.engine == ENGINE_C64) {
+        L.vec = want_vec;
+        LAUNCH(launch_cell64_pass(L));
+    } else if (kind == PASS_MOM && !plan.plain && mom_cells_supported(dp.P, dp.xs)) {
+        // (the shared-memory engine's plan: its runs of cells set the sums)
+        LAUNCH(launch_mom_cells(L, tiles * plan.GT));
     } else {
         LAUNCH(launch_gen_pass(L));
     }
@@ -1732,7 +1742,7 @@ void run_sandwich(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, con
         const int nseg = choose_nseg(ctx, dp, plan, tiles, form);
         PassBuffers pb = pass_buffers(ctx, PASS_SANDWICH, dp.P, (size_t)nseg * tiles * plan.GT);
         launch_pass(ctx, dp, PASS_SANDWICH, plan, nseg, tiles, dp.fine_bound,
-                    dp.fine_ptr, dp.nfine + 1, act, cnt, nullptr, pb, prm);
+                    dp.fine_ptr, dp.nfine + 1, act, cnt, nullptr, pb, prm, 0, nullptr, false, false);
         LAUNCH(launch_sandwich_finalize(pb.partWd(), nseg, tiles * plan.GT, dp.P, nullptr, 0, dp.n,
                                         act, cnt, (int)dp.G, bread, nullptr, nullptr, st));
         if (ctx->profiling) {

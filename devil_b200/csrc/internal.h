@@ -11,7 +11,7 @@
 namespace devil {
 
 enum PassKind { PASS_IRLS = 0, PASS_MOM = 1, PASS_MLE = 2, PASS_SANDWICH = 3 };
-enum Engine { ENGINE_REG = 0, ENGINE_GEN = 1, ENGINE_GRP = 2, ENGINE_TC = 3, ENGINE_TCW = 4 };
+enum Engine { ENGINE_REG = 0, ENGINE_GEN = 1, ENGINE_GRP = 2, ENGINE_TC = 3, ENGINE_TCW = 4, ENGINE_C64 = 5 };
 
 inline int pass_nw(PassKind k) { return k == PASS_MLE ? 3 : (k == PASS_MOM ? 0 : 1); }
 inline int pass_nv(PassKind k) { return (k == PASS_IRLS || k == PASS_SANDWICH) ? 1 : 0; }
@@ -44,6 +44,7 @@ struct PassLaunch {
     cudaStream_t stream;
     int* occ_out = nullptr;  // non-null: report the kernel's resident blocks per SM, launch nothing
     int plain = 0;           // the plain comparison form (FP32 staging in the shared-memory engine)
+    int vec = 1;             // bread pass: the score sums too (clusters); the FP64 matrix engine can leave them out
 };
 
 // engine choice helpers
@@ -81,6 +82,15 @@ int64_t tc_zimg_float4s(int64_t n);  // its size in float4
 cudaError_t launch_tc_zimg(const float* Xrm, int xs, int64_t n, int P, float4* zimg, cudaStream_t st);
 cudaError_t launch_tc_pass(const PassLaunch& L, const float4* zimg);
 cudaError_t launch_gen_pass(const PassLaunch& L);
+
+// ---- FP64 per-cell passes on the FP64 matrix instruction (kernels_cell64.cu) ----
+int cell64_tile_genes();
+bool cell64_supported(PassKind k, int P, int xs);
+cudaError_t launch_cell64_pass(const PassLaunch& L);
+// MOM moments with the sums of gen_pass_kernel<PassMOM> bit for bit (the same
+// runs of cells, each gene's terms added in cell order)
+bool mom_cells_supported(int P, int xs);
+cudaError_t launch_mom_cells(const PassLaunch& L, int max_slots);
 
 // ---- tensor-core IRLS engine for p = 5..32 (kernels_tcw.cu) ----
 // Inputs built once per fit by launch_tcw_prepare: the counts as a dense
