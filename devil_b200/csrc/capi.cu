@@ -255,6 +255,7 @@ struct DevProblem {
     // image, feature rows, padded offsets), built by its first launch
     mutable TcwGeom tcw;
     mutable bool tcw_ready = false;
+    mutable bool tcw_zfits = false;
     mutable int tcw_fits = -1;  // the dense count image fits half of the free device memory (-1: not asked)
     int precision = DEVIL_PREC_FP32;  // DEVIL_PREC_*: tensor-core passes at p <= 4
     double* Xdrm = nullptr;  // row-major FP64 copy for the FP64 passes
@@ -531,6 +532,8 @@ bool tcw_fits(const DevProblem& dp) {
         const double need = (double)dp.G * tcw_npad(dp.n) * (dp.val_u16 ? 2.0 : 4.0) +
                             (double)(dp.xs + 1) * tcw_npad(dp.n) * 4.0;
         dp.tcw_fits = need <= 0.5 * (double)fr ? 1 : 0;
+        // (with the products' image when that fits too)
+        dp.tcw_zfits = need + (double)tcw_zimg_bytes(dp.P, dp.n) <= 0.5 * (double)fr;
     }
     return dp.tcw_fits == 1;
 }
@@ -1250,6 +1253,7 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
                                   : (const void*)ws<float>(ctx, "tcw_y", (size_t)dp.G * t.ld);
             t.xt = ws<float>(ctx, "tcw_xt", (size_t)dp.xs * t.npad);
             t.offp = ws<float>(ctx, "tcw_off", (size_t)t.npad);
+            if (dp.tcw_zfits) t.zimg = ws<float>(ctx, "tcw_z", tcw_zimg_bytes(dp.P, dp.n) / sizeof(float));
             LAUNCH(launch_tcw_prepare(dp.rowptr, dp.col, dp.val, dp.val_u16, dp.G, dp.n, dp.Xrm, dp.xs,
                                       dp.off_f, t, ctx->stream));
             dp.tcw_ready = true;

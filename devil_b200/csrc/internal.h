@@ -101,6 +101,7 @@ struct TcwGeom {
     const float* xt = nullptr;
     const float* offp = nullptr;
     const void* ydense = nullptr;
+    const float* zimg = nullptr;  // split products of every chunk (tcw_zimg_bytes); null: formed in the pass
     int64_t ld = 0;
     int64_t npad = 0;
     int P = 0, NE = 0, NA = 0;
@@ -110,6 +111,7 @@ int tcw_blocks(int P);          // product blocks (grid.z)
 int tcw_tile_genes(PassKind k); // genes per tile: 128 (IRLS), 32 (MLE)
 int tcw_nblk(int P);
 int64_t tcw_npad(int64_t n);
+size_t tcw_zimg_bytes(int P, int64_t n);
 bool tcw_supported(int P, int xs);
 cudaError_t launch_tcw_prepare(const int64_t* rowptr, const int32_t* col, const void* val, int val_u16,
                                int64_t G, int64_t n, const float* Xrm, int xs, const float* off,

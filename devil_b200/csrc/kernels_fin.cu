@@ -9,16 +9,36 @@ namespace devil {
 
 static inline unsigned nblk(int64_t m, int t) { return (unsigned)((m + t - 1) / t); }
 
-// sums[a] = sum over segments of part[seg][slot][a]  (lanes split a)
+// sums[a] = sum over segments of part[seg][slot][a], in segment order (lanes
+// split a).  Eight segments of two outputs are loaded before they are added: the
+// last genes of a loop leave up to 300 segments, and one load per addition made
+// the step 75 us whatever the number of genes.
 template <class T>
 DEV void reduce_partials(const T* part, int nseg, int slot_stride, int slot, int stride, int count,
                          double* sums, int lane) {
-#pragma unroll 4
-    for (int a = lane; a < count; a += 32) {
-        double s = 0.0;
-        for (int seg = 0; seg < nseg; ++seg)
-            s += (double)part[((int64_t)seg * slot_stride + slot) * stride + a];
-        sums[a] = s;
+    constexpr int A = 2, U = 8;
+    const int64_t step = (int64_t)slot_stride * stride;
+    for (int a0 = lane; a0 < count; a0 += 32 * A) {
+        const T* p = part + (int64_t)slot * stride + a0;
+        double s[A];
+#pragma unroll
+        for (int j = 0; j < A; ++j) s[j] = 0.0;
+        for (int s0 = 0; s0 < nseg; s0 += U, p += U * step) {
+            T v[A][U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < A; ++j)
+                    v[j][u] = s0 + u < nseg && a0 + 32 * j < count ? __ldg(p + u * step + 32 * j) : T(0);
+#pragma unroll
+            for (int j = 0; j < A; ++j)
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (s0 + u < nseg) s[j] += (double)v[j][u];
+        }
+#pragma unroll
+        for (int j = 0; j < A; ++j)
+            if (a0 + 32 * j < count) sums[a0 + 32 * j] = s[j];
     }
 }
 

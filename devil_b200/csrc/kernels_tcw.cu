@@ -17,7 +17,9 @@
 // directly: the pass reads a dense image of the counts (gene rows of
 // npad cells, uint16 or float), so no separate nonzero pass is needed.
 //
-// Per chunk the CUDA cores compute eta = off + x beta (FP32, packed FMAs),
+// Per chunk the CUDA cores compute eta = off + x beta (FP32, packed FMAs; the
+// images hold a quad's cells in the order 0, 2, 1, 3, so that every pair that a
+// packed instruction takes is one register pair as loaded),
 // mu (ex2), r (rcp), the weights, and the chunk's products z = x_i x_j;
 // HW and Z enter as split TF32 pairs (v = hi + lo) and the MMA sums
 //     HW_hi Z_hi + HW_lo Z_hi + HW_hi Z_lo
@@ -51,7 +53,8 @@ namespace {
 
 constexpr int kWM = 128;                  // genes per tile: MMA M, tensor-memory lanes
 constexpr int kWKC = 32;                  // cells per chunk (4 K-steps of 8 TF32)
-constexpr int kWNT = 256;                 // threads per block
+constexpr int kWNT = 384;                 // threads per block: 256 of the weights, 128 of the products
+constexpr int kWW = 256;
 constexpr int kWNmax = 176;               // product columns per block at most
 constexpr int kWRun = 8;                  // chunks per tensor-memory run (256 cells)
 constexpr int kWA = kWM * kWKC * 4;       // one of HW_hi, HW_lo: 16 KB
@@ -70,14 +73,30 @@ constexpr int tcw_smem(int XS, int nblk) {
 static_assert(tcw_smem<float, false>(32, kWNmax) <= 227 * 1024, "stages fit the shared memory of one block");
 static_assert(tcw_smem<float, true>(32, kWNmax) <= 227 * 1024, "stages fit the shared memory of one block");
 
-// (a0, a1) += (b0, b1) * (c0, c1) as one packed FP32x2 FMA
-DEV void fma2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
-    uint64_t acc, bb, cc;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(acc) : "f"(a0), "f"(a1));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(bb) : "f"(b0), "f"(b1));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(cc) : "f"(c0), "f"(c1));
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(bb), "l"(cc));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(acc));
+// pairs of FP32 values in one 64-bit register pair
+DEV uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+DEV void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+// a + b * c, both halves (two correctly rounded FMAs)
+DEV uint64_t fma2(uint64_t b, uint64_t c, uint64_t a) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(c), "l"(a));
+    return r;
+}
+DEV uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a quad's four values of one feature: cells (0, 2) and (1, 3) as pairs (the
+// order the images are written in, tcw_quad_pos)
+DEV void ld_quad(const void* p, uint64_t& c02, uint64_t& c13) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    c02 = v.x;
+    c13 = v.y;
 }
 
 // counts of cells 4q..4q+3 of gene row gr in a count stage of R rows
@@ -126,9 +145,16 @@ DEV void store_split(unsigned char* sA, int row, int q, const float* v) {
     *reinterpret_cast<float4*>(sA + kWA + stage_off(row, q, kWM)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
 }
 
+// Threads 0..255 (the weights) form the weights of a chunk and the score;
+// threads 256..383 (the products) bring the inputs and the products (from the
+// image by bulk copies; formed here when the image does not fit the memory), add
+// finished runs into the total and issue the MMAs, so that the two halves of the
+// work overlap and one barrier per chunk is left.
 // The IRLS pass (MLE = false): 128 genes per tile, A row = gene, weight
-// r (1 + y / k); thread = (gene row tid % 128, cells of quads 4 h .. 4 h + 3
-// with h = tid / 128), the score in registers.
+// r (1 + y / k); weight thread = (gene row tid % 128, cells of quads 4 h .. 4 h
+// + 3 with h = tid / 128), the score in registers; up to 16 features a quad's
+// values stay in registers from eta to the score (one shared read each: 16-byte
+// reads that all lanes share take the register file's write bandwidth).
 // The dispersion pass (MLE = true; PassMLE in passes.cuh,
 // src/overdispersion.cpp:95-242): 32 genes per tile, A rows 32 b + gene
 // carry the Cox-Reid weights w, -w^2, 2 w^3 (b = 0, 1, 2; rows 96..127
@@ -139,7 +165,8 @@ template <int XS, class VT, bool MLE>
 __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassParamsAny prm, TcwGeom tw) {
     constexpr int GTn = MLE ? kMleG : kWM;
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ __align__(8) uint64_t bars[2];   // MMAs of the stage's chunk done
+    __shared__ __align__(8) uint64_t zbars[2];  // the stage's products in place (zimg)
     __shared__ uint32_t tslot;
     __shared__ int abort_flag;
     __shared__ int16_t ptab[kWNmax];  // product row -> i | j << 8 (-1: padding)
@@ -157,16 +184,23 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
     const uint32_t ncols = 2 * tot;                  // columns allocated
     const int tid = threadIdx.x, warp = tid >> 5;
     const int gi = tid & (GTn - 1);  // this thread's gene within the tile
-    const int hh = tid >> 7;         // IRLS: half of the chunk's cells (and of the drained columns)
+    const bool wt = tid < kWW;       // a weight thread
+    const int pt = tid - kWW;        // product thread
+    const int hh = (tid >> 7) & 1;   // IRLS: half of the chunk's cells (and of the last run's columns)
     const bool extra = zb == 0;      // block z = 0 adds the score / scalar sums
 
     int slot = tile * GTn + gi;
     const bool valid_slot = slot < nact;
     if (!valid_slot) slot = tile * GTn;  // duplicate a valid gene; not written
     const int g = __ldg(geo.act + slot);
-    float bt[XS];
+    uint64_t bt[XS];  // the coefficient, twice
+    if (wt) {
 #pragma unroll
-    for (int i = 0; i < XS; ++i) bt[i] = i < tw.P ? __ldg(prm.beta + (int64_t)g * tw.P + i) * kLog2e : 0.f;
+        for (int i = 0; i < XS; ++i) {
+            const float b = i < tw.P ? __ldg(prm.beta + (int64_t)g * tw.P + i) * kLog2e : 0.f;
+            bt[i] = pack2(b, b);
+        }
+    }
     float kk = 0.f, rk = 0.f, thf = 0.f;
     double theta = 0.0, aa = 0.0;
     if constexpr (MLE) {
@@ -225,10 +259,10 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
         }
     }
 
-    auto fetch = [&](int kc) {
+    auto fetch = [&](int kc) {  // (product threads)
         unsigned char* ib = in_slot(kc % kWRing);
         const int64_t cs = (k0 + kc) * kWKC;
-        for (int idx = tid; idx < XS * 8 + 8; idx += kWNT) {
+        for (int idx = pt; idx < XS * 8 + 8; idx += kWNT - kWW) {
             if (idx < XS * 8) {
                 const int i = idx >> 3, q = idx & 7;
                 cp_async<16>(ib + stage_off(i, q, XS), tw.xt + (int64_t)i * tw.npad + cs + 4 * q);
@@ -240,30 +274,28 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
         unsigned char* yb = ib + XS * kWKC * 4 + kWKC * 4;
         constexpr int CPP = 16 / (int)sizeof(VT);  // cells per piece
         constexpr int NPG = kWKC / CPP;            // pieces per gene row
-        if constexpr (MLE) {
-            // piece (gene tid % 32, p = tid / 32)
-            if (tid < kMleG * NPG) {
-                const int p = tid >> 5;
-                cp_async<16>(yb + (p * kMleG + gi) * 16, yrow + cs + p * CPP);
-            }
-        } else {
+        // gene gi; IRLS: its whole row, MLE: every fourth piece from pt / 32
 #pragma unroll
-            for (int u = 0; u < NPG / 2; ++u) {
-                const int p = hh + 2 * u;  // piece index within the row
-                cp_async<16>(yb + (p * kWM + gi) * 16, yrow + cs + p * CPP);
-            }
+        for (int u = 0; u < (MLE ? NPG / 4 : NPG); ++u) {
+            const int p = MLE ? (pt >> 5) + 4 * u : u;
+            cp_async<16>(yb + (p * GTn + gi) * 16, yrow + cs + p * CPP);
         }
     };
 
-    if (nchunk > 0) fetch(0);
-    cp_async_commit();
-    if (nchunk > 1) fetch(1);
-    cp_async_commit();
+    if (!wt) {
+        if (nchunk > 0) fetch(0);
+        cp_async_commit();
+        if (nchunk > 1) fetch(1);
+        cp_async_commit();
+        cp_async_wait<1>();  // chunk 0 has landed
+    }
 
     if (tid == 0) {
         abort_flag = 0;
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
+        mbar_init(&zbars[0], 1);
+        mbar_init(&zbars[1], 1);
         mbar_fence_init();
     }
     if (warp == 0) {
@@ -283,142 +315,181 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
 
     // IRLS score: cells (0, 1) and (2, 3) of each quad; MLE: the FP32 and
     // FP64 scalar sums
-    float va[MLE ? 1 : XS], vb[MLE ? 1 : XS];
+    uint64_t vab[MLE ? 1 : XS];
     float fs[2] = {0.f, 0.f};
     double sc[4] = {0.0, 0.0, 0.0, 0.0};
     if constexpr (!MLE) {
 #pragma unroll
-        for (int i = 0; i < XS; ++i) va[i] = vb[i] = 0.f;
+        for (int i = 0; i < XS; ++i) vab[i] = 0;
     }
+
+    // the chunk's products of this block from the image: one bulk copy
+    const uint32_t zbytes = (uint32_t)(2 * nblk * kWKC * 4);
+    const unsigned char* zsrc =
+        tw.zimg ? reinterpret_cast<const unsigned char*>(tw.zimg) + ((int64_t)zb * (tw.npad / kWKC) + k0) * zbytes
+                : nullptr;
+    bool zlost = false;  // (thread kWW) a bulk copy did not arrive in time
 
     int issued = 0;   // chunks whose MMAs were committed (uniform)
     int drained = 0;  // runs added into the total (uniform)
     for (int k = 0; k < nchunk; ++k) {
         const int st = k & 1;
-        bool ok = true;
-        // chunk k - 2's MMAs have completed: operand stage st is free
-        if (k >= 2) ok = mbar_wait_bounded(&bars[st], (uint32_t)(((k - 2) >> 1) & 1));
-        if (!ok) atomicExch(&abort_flag, 1);
-        if (k + 2 < nchunk) fetch(k + 2);
-        cp_async_commit();
-        cp_async_wait<2>();  // this thread's copies of chunk k have landed
-        __syncthreads();     // ... and everyone's
-        if (abort_flag) break;
-
+        bool ok = !zlost;
+        // chunk k - 2's MMAs have completed: operand stage st is free.  (Chunk
+        // k's inputs: the last barrier.)
+        if (k >= 2) ok = mbar_wait_bounded(&bars[st], (uint32_t)(((k - 2) >> 1) & 1)) && ok;
         const unsigned char* ib = in_slot(k % kWRing);
-        const float4* x4 = reinterpret_cast<const float4*>(ib);
-        const float4* o4 = reinterpret_cast<const float4*>(ib + XS * kWKC * 4);
-        const VT* ys = reinterpret_cast<const VT*>(ib + XS * kWKC * 4 + kWKC * 4);
         unsigned char* sA = op(st);
-        // the weights of this thread's gene at its cells
+        if (wt && ok) {
+            const float4* o4 = reinterpret_cast<const float4*>(ib + XS * kWKC * 4);
+            const VT* ys = reinterpret_cast<const VT*>(ib + XS * kWKC * 4 + kWKC * 4);
+            // the weights of this thread's gene at its cells
+#pragma unroll(XS <= 16 ? 2 : 1)
+            for (int qi = 0; qi < (MLE ? 1 : 4); ++qi) {
+                const int q = MLE ? warp : 4 * hh + qi;
+                const float4 o = o4[q];  // cells 0, 2, 1, 3
+                uint64_t e02 = pack2(o.x * kLog2e, o.y * kLog2e), e13 = pack2(o.z * kLog2e, o.w * kLog2e);
+                constexpr bool KEEP = !MLE && XS <= 16;
+                uint64_t xa[KEEP ? XS : 1], xb[KEEP ? XS : 1];
 #pragma unroll
-        for (int qi = 0; qi < (MLE ? 1 : 4); ++qi) {
-            const int q = MLE ? warp : 4 * hh + qi;
-            const float4 o = o4[q];
-            float e0 = o.x * kLog2e, e1 = o.y * kLog2e, e2 = o.z * kLog2e, e3 = o.w * kLog2e;
+                for (int i = 0; i < XS; ++i) {
+                    uint64_t a, b;
+                    ld_quad(ib + stage_off(i, q, XS), a, b);
+                    e02 = fma2(bt[i], a, e02);
+                    e13 = fma2(bt[i], b, e13);
+                    if constexpr (KEEP) {
+                        xa[i] = a;
+                        xb[i] = b;
+                    }
+                }
+                float y[4];
+                load_counts<GTn>(ys, q, gi, y);
+                float e[4];
+                unpack2(e02, e[0], e[2]);
+                unpack2(e13, e[1], e[3]);
+                if constexpr (MLE) {
+                    float w1[4], w2[4], w3[4];
 #pragma unroll
-            for (int i = 0; i < XS; ++i) {
-                const float4 x = x4[q * XS + i];
-                fma_x2(e0, e1, bt[i], x.x, x.y);
-                fma_x2(e2, e3, bt[i], x.z, x.w);
-            }
-            float y[4];
-            load_counts<GTn>(ys, q, gi, y);
-            const float e[4] = {e0, e1, e2, e3};
-            if constexpr (MLE) {
-                float w1[4], w2[4], w3[4];
+                    for (int c = 0; c < 4; ++c) {
+                        const float mu = ex2_approx(e[c]);
+                        const float xx = mu * thf;
+                        const float r = rcp_r(1.f + xx);
+                        const float w = mu * r;
+                        w1[c] = w;
+                        w2[c] = -w * w;
+                        w3[c] = 2.f * w * w * w;
+                        if (extra) {
+                            fs[0] += nb_ll_term<float>(xx, r);
+                            fs[1] += w * xx * r;
+                            if (y[c] > 0.f) {
+                                const double m = mu, yy = y[c];
+                                const double den = 1.0 + m * theta;
+                                double rr = (double)rcp_approx((float)den);
+                                rr = rr + rr * (1.0 - den * rr);
+                                sc[0] += yy * theta * rr;
+                                sc[1] += yy * rr * rr;
+                                double d1, d2;
+                                psi_diffs_tab(yy, aa, tab, d1, d2);
+                                sc[2] += d1;
+                                sc[3] += d2;
+                            }
+                        }
+                    }
+                    store_split(sA, gi, q, w1);
+                    store_split(sA, 32 + gi, q, w2);
+                    store_split(sA, 64 + gi, q, w3);
+                } else {
+                    float hw[4], sw[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float mu = ex2_approx(e[c]);
-                    const float xx = mu * thf;
-                    const float r = rcp_r(1.f + xx);
-                    const float w = mu * r;
-                    w1[c] = w;
-                    w2[c] = -w * w;
-                    w3[c] = 2.f * w * w * w;
+                    for (int c = 0; c < 4; ++c) {
+                        const float mu = ex2_approx(e[c]);
+                        const float r = rcp_approx(mu + kk);
+                        const float yr = y[c] * r;
+                        hw[c] = fmaf(yr, rk, r);    // r + y r / k
+                        sw[c] = fmaf(mu, r, -yr);   // (mu - y) r
+                    }
+                    store_split(sA, gi, q, hw);
                     if (extra) {
-                        fs[0] += nb_ll_term<float>(xx, r);
-                        fs[1] += w * xx * r;
-                        if (y[c] > 0.f) {
-                            const double m = mu, yy = y[c];
-                            const double den = 1.0 + m * theta;
-                            double rr = (double)rcp_approx((float)den);
-                            rr = rr + rr * (1.0 - den * rr);
-                            sc[0] += yy * theta * rr;
-                            sc[1] += yy * rr * rr;
-                            double d1, d2;
-                            psi_diffs_tab(yy, aa, tab, d1, d2);
-                            sc[2] += d1;
-                            sc[3] += d2;
+                        const uint64_t s02 = pack2(sw[0], sw[2]), s13 = pack2(sw[1], sw[3]);
+#pragma unroll
+                        for (int i = 0; i < XS; ++i) {
+                            uint64_t a, b;
+                            if constexpr (KEEP) {
+                                a = xa[i];
+                                b = xb[i];
+                            } else {
+                                ld_quad(ib + stage_off(i, q, XS), a, b);
+                            }
+                            vab[i] = fma2(s02, a, vab[i]);
+                            vab[i] = fma2(s13, b, vab[i]);
                         }
                     }
                 }
-                store_split(sA, gi, q, w1);
-                store_split(sA, 32 + gi, q, w2);
-                store_split(sA, 64 + gi, q, w3);
-            } else {
-                float hw[4], sw[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float mu = ex2_approx(e[c]);
-                    const float r = rcp_approx(mu + kk);
-                    const float yr = y[c] * r;
-                    hw[c] = fmaf(yr, rk, r);    // r + y r / k
-                    sw[c] = fmaf(mu, r, -yr);   // (mu - y) r
-                }
-                store_split(sA, gi, q, hw);
-                if (extra) {
-#pragma unroll
-                    for (int i = 0; i < XS; ++i) {
-                        const float4 x = x4[q * XS + i];
-                        fma2(va[i], vb[i], sw[0], sw[2], x.x, x.z);
-                        fma2(va[i], vb[i], sw[1], sw[3], x.y, x.w);
-                    }
-                }
             }
-        }
-        // the chunk's products of this block, split
-        {
-            unsigned char* sB = sA + 2 * kWA;
-            int row = tid % nblk, q = tid / nblk;
-            for (; q < 8;) {
-                const int pr = ptab[row];
-                float4 hz = make_float4(0.f, 0.f, 0.f, 0.f), lz = hz;
-                if (pr >= 0) {
-                    const float4 xi = x4[q * XS + (pr & 0xFF)];
-                    const float4 xj = x4[q * XS + (pr >> 8)];
-                    tf32_split(xi.x * xj.x, hz.x, lz.x);
-                    tf32_split(xi.y * xj.y, hz.y, lz.y);
-                    tf32_split(xi.z * xj.z, hz.z, lz.z);
-                    tf32_split(xi.w * xj.w, hz.w, lz.w);
-                }
-                *reinterpret_cast<float4*>(sB + stage_off(row, q, nblk)) = hz;
-                *reinterpret_cast<float4*>(sB + nblk * kWKC * 4 + stage_off(row, q, nblk)) = lz;
-                row += kWNT;
+        } else if (!wt) {
+            if (tid == kWW && zsrc && ok) {
+                mbar_arrive_expect_tx(&zbars[st], zbytes);
+                bulk_g2s(sA + 2 * kWA, zsrc + (int64_t)k * zbytes, zbytes, &zbars[st]);
+            }
+            if (k + 2 < nchunk) fetch(k + 2);  // (its slot was read in chunk k - 1)
+            cp_async_commit();
+            // without the image: the chunk's products of this block, split
+            if (ok && !zsrc) {
+                unsigned char* sB = sA + 2 * kWA;
+                int row = pt, q = 0;
                 while (row >= nblk) {
                     row -= nblk;
                     ++q;
                 }
+                for (; q < 8;) {
+                    const int pr = ptab[row];
+                    float4 hz = make_float4(0.f, 0.f, 0.f, 0.f), lz = hz;
+                    if (pr >= 0) {
+                        uint64_t ia, ic, ja, jc;
+                        ld_quad(ib + stage_off(pr & 0xFF, q, XS), ia, ic);
+                        ld_quad(ib + stage_off(pr >> 8, q, XS), ja, jc);
+                        float z0, z1, z2, z3;
+                        unpack2(mul2(ia, ja), z0, z2);
+                        unpack2(mul2(ic, jc), z1, z3);
+                        tf32_split(z0, hz.x, lz.x);
+                        tf32_split(z1, hz.y, lz.y);
+                        tf32_split(z2, hz.z, lz.z);
+                        tf32_split(z3, hz.w, lz.w);
+                    }
+                    *reinterpret_cast<float4*>(sB + stage_off(row, q, nblk)) = hz;
+                    *reinterpret_cast<float4*>(sB + nblk * kWKC * 4 + stage_off(row, q, nblk)) = lz;
+                    row += kWNT - kWW;
+                    while (row >= nblk) {
+                        row -= nblk;
+                        ++q;
+                    }
+                }
             }
+            // chunk k - 1 closed a run: add it into the total once its MMAs
+            // have completed (the work above overlapped them)
+            if (k > 0 && k % kWRun == 0) {
+                bool okd = mbar_wait_bounded(&bars[(k - 1) & 1], (uint32_t)(((k - 1) >> 1) & 1));
+                okd = __all_sync(0xffffffffu, okd);
+                if (okd) {
+                    tc_fence_after();
+                    tcw_drain(tmem, lanes, tot, 0, nblk, drained == 0);
+                } else {
+                    ok = false;
+                }
+            }
+            cp_async_wait<1>();  // chunk k + 1 has landed
         }
+        if (k > 0 && k % kWRun == 0) ++drained;
         fence_async_smem();
-        // chunk k - 1 closed a run: add it into the total once its MMAs
-        // have completed (the work above overlapped them)
-        if (k > 0 && k % kWRun == 0) {
-            bool okd = mbar_wait_bounded(&bars[(k - 1) & 1], (uint32_t)(((k - 1) >> 1) & 1));
-            okd = __all_sync(0xffffffffu, okd);
-            if (okd) {
-                tc_fence_after();
-                tcw_drain(tmem, lanes, tot, dc0, dc1, drained == 0);
-            } else {
-                atomicExch(&abort_flag, 1);
-            }
-            ++drained;
-        }
         tc_fence_before();
-        __syncthreads();
-        if (abort_flag) break;
-        if (tid == 0) {
+        // operands of chunk k and inputs of chunk k + 1 are in place; every
+        // thread learns of a wait that gave up
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) abort_flag = 1;
+            break;
+        }
+        if (tid == kWW && zsrc && !mbar_wait_bounded(&zbars[st], (uint32_t)((k >> 1) & 1))) zlost = true;
+        if (tid == kWW && !zlost) {
             tc_fence_after();
             const uint32_t a_hi = smem_u32(sA), a_lo = a_hi + kWA;
             const uint32_t b_hi = a_hi + 2 * kWA, b_lo = b_hi + (uint32_t)(nblk * kWKC * 4);
@@ -447,14 +518,14 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
     tc_fence_after();
     __syncthreads();  // abort_flag is final from here on
     const bool good = !abort_flag;
-    if (good && issued > 0) tcw_drain(tmem, lanes, tot, dc0, dc1, drained == 0);  // the last run
+    if (wt && good && issued > 0) tcw_drain(tmem, lanes, tot, dc0, dc1, drained == 0);  // the last run
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
 
     // the Hessian-like columns of this warp's lanes: IRLS rows = genes;
     // MLE rows 32 b + gene (b = warp % 4 < 3)
-    {
+    if (wt) {
         const int b = MLE ? (warp & 3) : 0;
         const int lg = MLE ? (tid & 31) : gi;  // gene of this thread's tensor-memory lane
         const bool write = good && tile * GTn + lg < nact && (!MLE || b < 3);
@@ -482,10 +553,12 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
             // the 8 quads' sums of each gene, added in quad order
             float* fred = reinterpret_cast<float*>(smem);                  // [8][32][2]
             double* dred = reinterpret_cast<double*>(smem + 8 * 32 * 2 * 4);  // [8][32][4]
-            fred[(warp * 32 + gi) * 2 + 0] = fs[0];
-            fred[(warp * 32 + gi) * 2 + 1] = fs[1];
+            if (wt) {
+                fred[(warp * 32 + gi) * 2 + 0] = fs[0];
+                fred[(warp * 32 + gi) * 2 + 1] = fs[1];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dred[(warp * 32 + gi) * 4 + j] = sc[j];
+                for (int j = 0; j < 4; ++j) dred[(warp * 32 + gi) * 4 + j] = sc[j];
+            }
             __syncthreads();
             if (warp == 0 && write) {
                 float f0 = 0.f, f1 = 0.f;
@@ -506,15 +579,22 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
             // the two halves of the cells: half 1 hands its sums to half 0
             // through the (idle) first operand stage
             float* red = reinterpret_cast<float*>(smem);  // [128 genes][XS]
-            if (hh == 1) {
+            float v[XS];
 #pragma unroll
-                for (int i = 0; i < XS; ++i) red[gi * XS + i] = va[i] + vb[i];
+            for (int i = 0; i < XS; ++i) {
+                float a, b;
+                unpack2(vab[i], a, b);
+                v[i] = a + b;
+            }
+            if (wt && hh == 1) {
+#pragma unroll
+                for (int i = 0; i < XS; ++i) red[gi * XS + i] = v[i];
             }
             __syncthreads();
-            if (hh == 0 && write) {
+            if (wt && hh == 0 && write) {
 #pragma unroll
                 for (int i = 0; i < XS; ++i)
-                    if (i < tw.P) out[tw.NE + i] = va[i] + vb[i] + red[gi * XS + i];
+                    if (i < tw.P) out[tw.NE + i] = v[i] + red[gi * XS + i];
             }
         }
     }
@@ -564,7 +644,46 @@ __global__ void tcw_dense_kernel(const int64_t* __restrict__ rowptr, const int32
     }
 }
 
-// feature rows of the design (zero past n and past p) and the offsets:
+// The products of every chunk and block z as the MMA reads them: [z][chunk][hi,
+// lo][quad][row][4 cells], split as the kernel splits them.  Made once per fit:
+// forming them per tile cost the 128 product threads more instructions a chunk
+// than the weights cost the other 256 (8,500 genes x 30,000 cells, p = 16, first
+// IRLS pass: 1,479 us with the products formed in the kernel, 1,033 with the
+// image; first MLE pass 4,712 and 3,641).
+__global__ void tcw_zimg_kernel(const float* __restrict__ xt, int64_t npad, int NE, int nblk, int nz, float* z) {
+    const int64_t nch = npad / kWKC, total = (int64_t)nz * nch * nblk * 8;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int row = (int)(t % nblk);
+        const int64_t u = t / nblk;
+        const int q = (int)(u % 8);
+        const int64_t v = u / 8;  // z * nch + chunk
+        const int gp = (int)(v / nch) * nblk + row;
+        float4 hz = make_float4(0.f, 0.f, 0.f, 0.f), lz = hz;
+        if (gp < NE) {
+            int j = (int)((sqrtf(8.f * (float)gp + 1.f) - 1.f) * 0.5f);
+            while (j * (j + 1) / 2 > gp) --j;
+            while ((j + 1) * (j + 2) / 2 <= gp) ++j;
+            const int i = gp - j * (j + 1) / 2;
+            const int64_t c = (v % nch) * kWKC + 4 * q;
+            const float4 a = __ldg(reinterpret_cast<const float4*>(xt + (int64_t)i * npad + c));
+            const float4 b = __ldg(reinterpret_cast<const float4*>(xt + (int64_t)j * npad + c));
+            tf32_split(a.x * b.x, hz.x, lz.x);  // (xt holds cells 0, 2, 1, 3)
+            tf32_split(a.z * b.z, hz.y, lz.y);
+            tf32_split(a.y * b.y, hz.z, lz.z);
+            tf32_split(a.w * b.w, hz.w, lz.w);
+        }
+        unsigned char* o = reinterpret_cast<unsigned char*>(z) + v * (2 * nblk * kWKC * 4);
+        *reinterpret_cast<float4*>(o + stage_off(row, q, nblk)) = hz;
+        *reinterpret_cast<float4*>(o + nblk * kWKC * 4 + stage_off(row, q, nblk)) = lz;
+    }
+}
+
+// place of cell c in its quad: 0, 2, 1, 3 (the pairs of ld_quad)
+DEV int64_t tcw_quad_pos(int64_t c) { return (c & ~(int64_t)3) | ((c & 1) << 1) | ((c >> 1) & 1); }
+
+// feature rows of the design (zero past n and past p) and the offsets, the cells
+// of a quad in the order of tcw_quad_pos:
 // -1e30 past n, so that mu = 0 there and the padding cells of the last
 // chunk add nothing to any sum (the products and the score vanish with
 // x = 0 as well, the dispersion pass's scalar sums only with mu = 0)
@@ -574,8 +693,9 @@ __global__ void tcw_xt_kernel(const float* __restrict__ Xrm, int xs, int64_t n, 
          t += (int64_t)gridDim.x * blockDim.x) {
         const int i = (int)(t / npad);
         const int64_t c = t - (int64_t)i * npad;
-        if (i < xs) xt[t] = c < n ? Xrm[c * xs + i] : 0.f;
-        else offp[c] = c < n ? off[c] : -1e30f;
+        const int64_t at = tcw_quad_pos(c);
+        if (i < xs) xt[(int64_t)i * npad + at] = c < n ? Xrm[c * xs + i] : 0.f;
+        else offp[at] = c < n ? off[c] : -1e30f;
     }
 }
 
@@ -652,7 +772,13 @@ cudaError_t launch_tcw_prepare(const int64_t* rowptr, const int32_t* col, const 
     const int64_t tot = (int64_t)(xs + 1) * tw.npad;
     tcw_xt_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 148 * 16), 256, 0, st>>>(
         Xrm, xs, n, tw.npad, off, const_cast<float*>(tw.xt), const_cast<float*>(tw.offp));
+    if (tw.zimg)
+        tcw_zimg_kernel<<<148 * 16, 256, 0, st>>>(tw.xt, tw.npad, tw.NE, tw.nblk, tcw_blocks(tw.P),
+                                                  const_cast<float*>(tw.zimg));
     return cudaGetLastError();
+}
+size_t tcw_zimg_bytes(int P, int64_t n) {
+    return (size_t)tcw_blocks(P) * (size_t)(tcw_npad(n) / kWKC) * (size_t)(2 * tcw_nblk(P) * kWKC * 4);
 }
 
 int tcw_tile_genes(PassKind k) { return k == PASS_MLE ? kMleG : kWM; }
