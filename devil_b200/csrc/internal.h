@@ -361,7 +361,7 @@ cudaError_t launch_init_beta(const int64_t* rowptr, const int32_t* col, const vo
                              int val_u16, const double* Xrm, int xs, const double* off,
                              double* inv_sf, const double* ginv, const double* stats, int64_t G,
                              int64_t n, int P, int rough, double* beta, float* beta_f,
-                             cudaStream_t st);
+                             cudaStream_t st, const int32_t* order = nullptr);
 cudaError_t launch_segptr(const int64_t* rowptr, const int32_t* col, int64_t G,
                           const int32_t* bound, int nbound, int64_t* segptr, cudaStream_t st);
 cudaError_t launch_validate_csr(const int64_t* rowptr, const int32_t* col, int64_t G, int64_t n,

@@ -472,8 +472,8 @@ cudaError_t run_bread(const PassLaunch& L) {
 }  // namespace
 
 int cell64_tile_genes() { return kCG; }
-// (row strides of 4, 8, 12, .. doubles; measured above the register engine's p)
-bool cell64_supported(PassKind k, int P, int xs) { return k == PASS_SANDWICH && P > 8 && P <= 32 && xs % 4 == 0; }
+// (row strides of 4, 8, 12, .. doubles)
+bool cell64_supported(PassKind k, int P, int xs) { return k == PASS_SANDWICH && P >= 3 && P <= 32 && xs % 4 == 0; }
 cudaError_t launch_cell64_pass(const PassLaunch& L) {
     if (!cell64_supported(L.kind, L.P, L.xs_pad)) return cudaErrorInvalidValue;
     return L.vec ? run_bread<true>(L) : run_bread<false>(L);

@@ -862,15 +862,19 @@ cudaError_t launch_xtx_inverse(const double* Xcm, int64_t n, int P, double* part
 // beta_0 (warp per gene).  QR least squares of log1p(y / exp(off)) on X:
 // the solution equals (X'X)^-1 X' z; z is zero wherever y is zero, so
 // X' z is a sum over the nonzero entries of the row.  Rough init:
-// beta_0 = (log1p(mean y), 0, ..., 0).
+// beta_0 = (log1p(mean y), 0, ..., 0).  U entries a lane are in flight and are
+// added in order; the genes with the most entries are taken first (one entry at
+// a time, a gene seen in every cell held its warp for 3,000 dependent rounds:
+// 10,000 x 100,000, p = 4: 3.59 -> 2.18 ms).
 template <class VT, int PMAX>
 __global__ void init_beta_kernel(const int64_t* rowptr, const int32_t* col, const VT* val,
                                  const double* Xrm, int xs, const double* inv_sf,
                                  const double* ginv, const double* stats, int64_t G, int64_t n,
-                                 int P, int rough, double* beta, float* beta_f) {
+                                 int P, int rough, double* beta, float* beta_f, const int32_t* order) {
     int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (g >= G) return;
+    if (order) g = order[g];
     if (rough) {
         if (lane < P) {
             double b = lane == 0 ? log1p(stats[g * 6 + 0]) : 0.0;
@@ -882,13 +886,47 @@ __global__ void init_beta_kernel(const int64_t* rowptr, const int32_t* col, cons
     double r[PMAX];
 #pragma unroll
     for (int i = 0; i < PMAX; ++i) r[i] = 0.0;
-    for (int64_t e = rowptr[g] + lane; e < rowptr[g + 1]; e += 32) {
-        int c = col[e];
-        double z = log1p((double)val[e] * inv_sf[c]);
-        const double* xr = Xrm + (int64_t)c * xs;
+    constexpr int U = PMAX <= 8 ? 8 : 4;    // entries in flight
+    constexpr int V = PMAX <= 4 ? 8 : (PMAX <= 8 ? 4 : (PMAX <= 16 ? 2 : 1));  // design rows in flight
+    const int64_t e1 = rowptr[g + 1];
+    int cn[U];
+    VT vn[U];
+    auto load_step = [&](int64_t eb) {
 #pragma unroll
-        for (int i = 0; i < PMAX; ++i)
-            if (i < P) r[i] += xr[i] * z;
+        for (int u = 0; u < U; ++u) {
+            const int64_t e = eb + 32 * u;
+            cn[u] = e < e1 ? __ldg(col + e) : -1;
+            vn[u] = e < e1 ? val[e] : VT(0);
+        }
+    };
+    load_step(rowptr[g] + lane);
+    for (int64_t eb = rowptr[g] + lane; eb < e1; eb += 32 * U) {
+        int c[U];
+        double z[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            c[u] = cn[u];
+            z[u] = c[u] >= 0 ? (double)vn[u] * __ldg(inv_sf + c[u]) : 0.0;
+        }
+        load_step(eb + 32 * U);
+#pragma unroll
+        for (int u0 = 0; u0 < U; u0 += V) {
+            double x[V][PMAX];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const double* xr = Xrm + (int64_t)(c[u0 + v] >= 0 ? c[u0 + v] : 0) * xs;
+#pragma unroll
+                for (int i = 0; i < PMAX; ++i) x[v][i] = i < P ? __ldg(xr + i) : 0.0;
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                if (c[u0 + v] < 0) continue;
+                const double l = log1p(z[u0 + v]);
+#pragma unroll
+                for (int i = 0; i < PMAX; ++i)
+                    if (i < P) r[i] += x[v][i] * l;
+            }
+        }
     }
 #pragma unroll
     for (int i = 0; i < PMAX; ++i)
@@ -913,7 +951,7 @@ cudaError_t launch_init_beta(const int64_t* rowptr, const int32_t* col, const vo
                              int val_u16, const double* Xrm, int xs, const double* off,
                              double* inv_sf, const double* ginv, const double* stats, int64_t G,
                              int64_t n, int P, int rough, double* beta, float* beta_f,
-                             cudaStream_t st) {
+                             cudaStream_t st, const int32_t* order) {
     if (G == 0) return cudaSuccess;
     if (!rough) {
         inv_exp_kernel<<<(unsigned)std::min<int64_t>(nblk(n, 256), 1024), 256, 0, st>>>(off, n, inv_sf);
@@ -923,11 +961,11 @@ cudaError_t launch_init_beta(const int64_t* rowptr, const int32_t* col, const vo
     if (val_u16)                                                                                 \
         init_beta_kernel<uint16_t, PM><<<b, 256, 0, st>>>(rowptr, col, (const uint16_t*)val, Xrm, \
                                                             xs, inv_sf, ginv, stats, G, n, P,     \
-                                                            rough, beta, beta_f);                \
+                                                            rough, beta, beta_f, order);         \
     else                                                                                         \
         init_beta_kernel<float, PM><<<b, 256, 0, st>>>(rowptr, col, (const float*)val, Xrm, xs,   \
                                                          inv_sf, ginv, stats, G, n, P, rough,     \
-                                                         beta, beta_f);
+                                                         beta, beta_f, order);
     if (P <= 4) {
         DEVIL_INIT(4)
     } else if (P <= 8) {

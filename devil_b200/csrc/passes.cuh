@@ -568,25 +568,23 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
             }
         }
     } else {
-        // software pipeline: the next cell's row is in flight while the gene
-        // tile works on the current one
-        int c = c0 + threadIdx.x;
-        float xn[P];
-        float on = 0.f;
-        if (c < c1) {
-            load_row<P, PP>(geo.X, c, xn);
-            on = __ldg(geo.off + c);
-        }
-        for (; c < c1; c += NT) {
+        // software pipeline: the next two cells' rows are in flight while the
+        // gene tile works on the current one (one row ahead left most of an L2
+        // round trip exposed)
+        float xn[2][P];
+        float on[2] = {0.f, 0.f};
+        auto load_cell = [&](int c, int s) {
+            if (c < c1) {
+                load_row<P, PP>(geo.X, c, xn[s]);
+                on[s] = __ldg(geo.off + c);
+            }
+        };
+        auto cell = [&](int c, int s) {
             float x[P];
 #pragma unroll
-            for (int i = 0; i < P; ++i) x[i] = xn[i];
-            const float o = on * kLog2e;
-            const int cn = c + NT;
-            if (cn < c1) {
-                load_row<P, PP>(geo.X, cn, xn);
-                on = __ldg(geo.off + cn);
-            }
+            for (int i = 0; i < P; ++i) x[i] = xn[s][i];
+            const float o = on[s] * kLog2e;
+            load_cell(c + 2 * NT, s);
             float zz[P * (P + 1) / 2];
 #pragma unroll
             for (int jj = 0; jj < P; ++jj)
@@ -610,7 +608,15 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
                 RegAcc<P, NAc, NSc, AW, AS, float> acc{aw[j], as[j], x, zz};
                 Pass::template dense<float>(gp[j], mu, acc);
             }
+        };
+        int c = c0 + threadIdx.x;
+        load_cell(c, 0);
+        load_cell(c + NT, 1);
+        for (; c + NT < c1; c += 2 * NT) {
+            cell(c, 0);
+            cell(c + NT, 1);
         }
+        if (c < c1) cell(c, 0);
     }
     // sparse corrections: UNR independent nonzeros per thread per step, so
     // their dependent (index -> design row) loads overlap
