@@ -1044,8 +1044,7 @@ struct PassPlan {
     int GT;
     PassKind kind = PASS_IRLS;
     int plain = 0;  // the plain comparison form
-    int waves = 0;  // design groups: waves of a slice-major step; wide tensor cores: minimum waves
-                    // (0: the engine's default)
+    int waves = 0;  // wide tensor cores: minimum waves (0: the engine's default)
 };
 
 // the tensor-core IRLS engine for p = 5..32 (kernels_tcw.cu): DEVIL_TCW=1
@@ -1229,7 +1228,7 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
             if (kind == PASS_MLE) gg.psitab = ws<double>(ctx, "grp_psitab", (size_t)tiles * kGrpTab);
             // (the IRLS step folds the assembly into its finalize)
             LAUNCH(launch_grp_slices(kind, gg, prm, dp.val_u16, tiles,
-                                     grp_slices_tile(tiles, gg.S, ctx->sm_count, plan.waves > 0 ? plan.waves : 3),
+                                     grp_slices_tile(tiles, gg.S, dp.n, ctx->sm_count),
                                      kind != PASS_IRLS,
                                      ctx->stream, rowexp_fresh));
         } else {
@@ -1341,16 +1340,15 @@ const int32_t* all_genes(devil_ctx* ctx, const DevProblem& dp, int32_t** count_o
 // tile autotuner
 // ------------------------------------------------------------------
 // Each engine has a tile knob whose best value depends on the shape: genes
-// per thread of the register engine (GT), the waves a slice-major step of
-// the design-group engine is spread over (its gene tile), the minimum
-// waves of the wide tensor-core pass (its cell segments).  On the first
+// per thread of the register engine (GT), the minimum waves of the wide
+// tensor-core pass (its cell segments).  (The design-group engine's tile follows
+// the active genes: grp_slices_tile.)  On the first
 // loop of a shape bucket (pass kind, engine, p, count type, log2 n,
 // log2 G, half-octaves of the density) in this process, each candidate
 // plan runs the loop's first pass once untimed and three times timed (CUDA
 // events on the context stream, all genes active); the fastest is kept for the
-// bucket.  The candidates leave every gene's result unchanged except for
-// the register and wide engines, whose FP32 segment sums can round
-// differently (well inside the parity bars).  DEVIL_AUTOTUNE=0 keeps the
+// bucket.  The candidates' FP32 segment sums can round differently (well
+// inside the parity bars).  DEVIL_AUTOTUNE=0 keeps the
 // heuristic defaults.
 struct TuneKey {
     int kind, engine, P, u16, nb, gb, db;
@@ -1366,7 +1364,7 @@ bool autotune_enabled() {
     return !(e && *e && atoi(e) == 0);
 }
 
-std::vector<PassPlan> tune_candidates(devil_ctx* ctx, const DevProblem& dp, const PassPlan& base) {
+std::vector<PassPlan> tune_candidates(const DevProblem& dp, const PassPlan& base) {
     std::vector<PassPlan> c{base};
     if (base.plain) return c;
     if (base.engine == ENGINE_REG && (base.kind == PASS_IRLS || base.kind == PASS_MLE)) {
@@ -1376,15 +1374,6 @@ std::vector<PassPlan> tune_candidates(devil_ctx* ctx, const DevProblem& dp, cons
             PassPlan p = base;
             p.GT = gt;
             c.push_back(p);
-        }
-    } else if (base.engine == ENGINE_GRP) {
-        const int bit = base.kind == PASS_IRLS ? 1 : (base.kind == PASS_MLE ? 2 : 0);
-        if (ctx->grp_slices & bit) {
-            for (int w : {2, 6}) {
-                PassPlan p = base;
-                p.waves = w;
-                c.push_back(p);
-            }
         }
     } else if (base.engine == ENGINE_TCW) {
         PassPlan p = base;
@@ -1405,7 +1394,7 @@ PassPlan autotune(devil_ctx* ctx, const DevProblem& dp, const PassPlan& base, co
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) return it->second;
-    const std::vector<PassPlan> cands = tune_candidates(ctx, dp, base);
+    const std::vector<PassPlan> cands = tune_candidates(dp, base);
     PassPlan best = base;
     if (cands.size() > 1) {
         const int was_profiling = ctx->profiling;
@@ -1414,8 +1403,7 @@ PassPlan autotune(devil_ctx* ctx, const DevProblem& dp, const PassPlan& base, co
         CK(cudaEventCreate(&t0));
         CK(cudaEventCreate(&t1));
         // once untimed, then the fastest of three rounds over the candidates in
-        // turn: one run each let a clock step or a neighbour's traffic pick a plan
-        // 10 % slower (4,000 genes x 1 M cells, p = 2: 41 to 47 ms a fit)
+        // turn: with one run each a clock step could pick the plan
         std::vector<float> ms(cands.size(), INFINITY);
         for (int rep = 0; rep < 4; ++rep)
             for (size_t i = 0; i < cands.size(); ++i) {
@@ -1950,7 +1938,7 @@ void fit_pipeline(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
         gg.rowexp = ws<double>(ctx, "grp_rowexp", (size_t)G * gg.U);
         double* zb = ws<double>(ctx, "grp_zero_beta", (size_t)G * P);
         CK(cudaMemsetAsync(zb, 0, (size_t)G * P * sizeof(double), st));
-        LAUNCH(launch_grp_init_beta(gg, dp.val_u16, zb, ginv, G, grp_slices_tile(G, gg.S, ctx->sm_count),
+        LAUNCH(launch_grp_init_beta(gg, dp.val_u16, zb, ginv, G, grp_slices_tile(G, gg.S, dp.n, ctx->sm_count),
                                     fb.beta, fb.beta_f, st));
     }
     else

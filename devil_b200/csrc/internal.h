@@ -261,7 +261,7 @@ cudaError_t launch_grp_pass(PassKind kind, const GrpGeom& geo, const PassParamsA
 // p x p sums (geo.gsum: slots x S x grp_slices_nq(kind) doubles;
 // geo.rowexp: G x U exp(x_u . beta) by gene, recomputed first unless
 // rowexp_fresh; geo.psitab, MLE: slots x kGrpTab)
-int grp_slices_tile(int64_t hint, int S, int sm_count, int waves = 3);
+int grp_slices_tile(int64_t hint, int S, int64_t n, int sm_count);
 // key[g] = entries of gene g, idx[g] = g (sorted descending into the work
 // order of the slice-major passes)
 cudaError_t launch_gene_entries(const int64_t* rowptr, int64_t G, int32_t* key, int32_t* idx,

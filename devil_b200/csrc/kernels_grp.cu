@@ -1241,25 +1241,36 @@ cudaError_t launch_gene_entries(const int64_t* rowptr, int64_t G, int32_t* key, 
     return cudaGetLastError();
 }
 
-int grp_slices_tile(int64_t hint, int S, int sm_count, int waves) {
-    // one resident block per SM (1,024 threads at 64 registers, the 128 KB
-    // slice stage); about `waves` waves (3 unless tuned), the tile count
-    // chosen so the last wave is nearly full, tiles of 16..1024 genes
-    const int64_t cap = (int64_t)sm_count;
-    int64_t tiles = std::max<int64_t>(1, ((int64_t)std::max(1, waves) * cap + S - 1) / S);
-    double best_eff = 0.0;
-    int64_t best = tiles;
-    for (int64_t tc = tiles; tc <= 2 * tiles; ++tc) {
-        const double waves = (double)tc * S / (double)cap;
-        const double eff = waves / std::ceil(waves);
-        if (eff > best_eff + 1e-9) {
-            best_eff = eff;
+// Genes per block of a slice-major pass over `hint` genes.  One block is
+// resident per SM (1,024 threads at 64 registers, the 128 KB slice stage), so a
+// grid of S x tc blocks runs in waves; each wave costs an SM its launch, the
+// stage and a tail, about as long as kWaveItems (gene, slice) items of a full
+// slice take (more of a small slice's, whose items are cheaper), and a last wave
+// that is not full costs its empty SMs.  With many genes active several
+// full waves win, with few one wave does.  A fixed count of waves, tuned on the
+// first pass, cost the late iterations (IRLS per fit at 1 / 2 / 3 / 6 waves:
+// 4,000 x 1 M, p = 2: 25.8 / 25.4 / 30.1 / 31.8 ms, by this rule 25.1; 4,000 x
+// 500,000, p = 12: 17.8 / 19.1 / 20.8 / 24.1, 17.3; 10,000 x 1 M, p = 32: 65.8 /
+// 65.1 / 66.1 / 69.8, 61.0; 3,001 x 20,011 in 154 slices: 10.0 / 10.4 / 11.0 /
+// 12.6, 9.9).
+constexpr double kWaveItems = 25.0;
+int grp_slices_tile(int64_t hint, int S, int64_t n, int sm_count) {
+    const double cap = (double)sm_count;
+    const double cells = (double)n / S;
+    const double wave = kWaveItems * (0.5 + 0.5 * cells / kSliceCells) * (kSliceCells + 2500.0) / (cells + 2500.0);
+    const double items = (double)hint * S / cap;  // per SM
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>((hint + 7) / 8, ((int64_t)8 * sm_count + S - 1) / S));
+    double best_cost = 0.0;
+    int64_t best = 1;
+    for (int64_t tc = 1; tc <= most; ++tc) {
+        const double waves = (double)tc * S / cap, whole = std::ceil(waves);
+        const double cost = whole * wave + items * whole / waves;
+        if (tc == 1 || cost < best_cost) {
+            best_cost = cost;
             best = tc;
         }
-        if (eff >= 0.95) break;
     }
-    const int64_t tile = (hint + best - 1) / best;
-    return (int)std::max<int64_t>(16, std::min<int64_t>(1024, tile));
+    return (int)((hint + best - 1) / best);
 }
 
 template <class Pass>
