@@ -802,7 +802,8 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     CK(cudaStreamSynchronize(st));
     int32_t* hist = ws<int32_t>(ctx, "grp_hist", (size_t)std::max<int64_t>(nsegs, 1) * NSL);
     LAUNCH(launch_group_csr(dp.rowptr, dp.col, dp.val, dp.val_u16, dp.G, segbase, S, cslice, cloc,
-                            NSL, hist, nsegs, gptr, gent, st));
+                            NSL, hist, ws<int32_t>(ctx, "grp_seggene", std::max<int64_t>(nsegs, 1)), nsegs, U,
+                            gptr, gent, st));
     if (NF > 0) {
         auto& gr = dp.grp;
         auto up = [&](const char* nm, const std::vector<int32_t>& v) {

@@ -316,7 +316,7 @@ cudaError_t launch_group_segments(const int64_t* rowptr, int64_t G, int S, int64
 // scatter); gent: GrpEnt entries
 cudaError_t launch_group_csr(const int64_t* rowptr, const int32_t* col, const void* val, int val_u16,
                              int64_t G, const int64_t* segbase, int S, const int32_t* ckey,
-                             const int32_t* cloc, int K, int32_t* hist, int64_t nsegs,
+                             const int32_t* cloc, int K, int32_t* hist, int32_t* seggene, int64_t nsegs, int rows,
                              int64_t* gptr, void* gent, cudaStream_t st);
 
 // ---- preparation kernels (kernels_prep.cu) ----
