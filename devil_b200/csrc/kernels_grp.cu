@@ -677,23 +677,43 @@ struct GrpAcc {
 
 constexpr int kGrpUnr = 8;          // entries per lane per batch of the nonzero loop
 constexpr int kGrpChunk = 2048;     // nonzeros per work unit (at least)
+// Lanes per work unit of the clustered bread/meat: a unit there is one piece of a
+// slice (a cluster's cells) or one rule of up to 20 nodes, a few tens of terms, and
+// a whole warp spent it on the row's exponential and on five steps of shuffles per
+// sum.  4,000 genes x 500,000 cells, 22 design rows x 40 clusters: the bread and
+// meat 4.3 ms with 32 lanes, 2.35 with 8, 2.06 with 4; in 3 clusters 0.9 with
+// either.  The other passes run here only when the slice-major kernels are off.
+constexpr int kGrpPartLanes = 4;
 constexpr int kGrpUnitsMax = 128;   // chunks beyond one per slice, per gene
 
-// x_u . beta over the nonzero entries of design row u (warp-wide sum)
-DEV double row_dot(const GrpGeom& geo, int u, const double* bet, int lane) {
+// sum over the LW lanes of a part of a warp (mask: those lanes), in all of them
+template <int LW>
+DEV double part_sum(double v, unsigned mask) {
+    if constexpr (LW == 32) {
+        return warp_sum(v);
+    } else {
+#pragma unroll
+        for (int o = LW / 2; o; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+}
+
+// x_u . beta over the nonzero entries of design row u (summed over LW lanes)
+template <int LW = 32>
+DEV double row_dot(const GrpGeom& geo, int u, const double* bet, int lane, unsigned mask = 0xffffffffu) {
     double a = 0.0;
     const int r1 = __ldg(geo.rptr + u + 1);
-    for (int e = __ldg(geo.rptr + u) + lane; e < r1; e += 32) a += __ldg(geo.rval + e) * bet[__ldg(geo.rcol + e)];
-    return warp_sum(a);
+    for (int e = __ldg(geo.rptr + u) + lane; e < r1; e += LW) a += __ldg(geo.rval + e) * bet[__ldg(geo.rcol + e)];
+    return part_sum<LW>(a, mask);
 }
 
 // The design-group pass, block per gene (MOM, MLE, bread/meat; the IRLS
 // pass runs slice-major, grp_irls_slices_kernel).  Work units of a gene:
 // one "rule unit" per group q (the zero-count terms of the group's cells
 // from its Gauss rule), then the gene's nonzeros slice by slice in chunks of
-// at least kGrpChunk entries.  Warps take units round robin; the group sums
-// are then formed in unit order (deterministic) and assembled.
-template <class Pass, class VT>
+// at least kGrpChunk entries.  Warps (parts of LW lanes of them) take units round
+// robin; the group sums are then formed in unit order (deterministic) and assembled.
+template <class Pass, class VT, int LW>
 __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pass::Params prm) {
     using Ent = GrpEnt<VT>;
     using ET = typename Ent::T;
@@ -732,12 +752,12 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
         gpar.tab.pa = digamma_d(gpar.a);
         gpar.tab.ta = trigamma_d(gpar.a);
     }
-    const int warp = t >> 5, lane = t & 31, nw = nt >> 5;
+    const int warp = t >> 5, lane = t & 31;
     const ET* __restrict__ gent = static_cast<const ET*>(geo.gent);
     const int64_t* gp = (pieces ? geo.f_ptr : geo.gptr) + (int64_t)g * (S + 1);
     // chunk size grows with the gene's nonzeros so that there are at most
     // S + kGrpUnitsMax nonzero units
-    const int64_t CH = max((int64_t)kGrpChunk, (gp[S] - gp[0] + kGrpUnitsMax - 1) / kGrpUnitsMax);
+    const int64_t CH = max((int64_t)(kGrpChunk / 32 * LW), (gp[S] - gp[0] + kGrpUnitsMax - 1) / kGrpUnitsMax);
     if (warp == 0) {
         int run = 0;
         for (int base = 0; base < S; base += 32) {
@@ -760,7 +780,9 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
     }
     __syncthreads();
     const int nunits = NGq + sstart[S];
-    for (int un = warp; un < nunits; un += nw) {
+    const int sub = t / LW, ln = t % LW, nsub = nt / LW;
+    const unsigned mask = LW == 32 ? 0xffffffffu : ((1u << (LW & 31)) - 1u) << (lane & ~(LW - 1));
+    for (int un = sub; un < nunits; un += nsub) {
         GrpAcc<NWV, NS> acc;
         acc.zero();
         if (un < NGq) {
@@ -768,9 +790,9 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
             const int q = un;
             const int u = geo.fine ? q / C : q;
             const int ri = (geo.fine && C > 1) ? U + q : u;  // C == 1: fine == coarse
-            const double A = exp(row_dot(geo, u, bet, lane));
+            const double A = exp(row_dot<LW>(geo, u, bet, ln, mask));
             const int m = __ldg(geo.rm + ri);
-            for (int j = lane; j < m; j += 32) {
+            for (int j = ln; j < m; j += LW) {
                 acc.q = __ldg(geo.rw + (int64_t)ri * kRuleCap + j);
                 const double mu = A * __ldg(geo.res + (int64_t)ri * kRuleCap + j);
                 Pass::template dense<double>(gpar, mu, acc);
@@ -789,29 +811,29 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
             }
             const int jc = cu - sstart[sl];
             const int u = __ldg(skey + sl) / (pieces ? C : 1);
-            const double A = exp(row_dot(geo, u, bet, lane));
+            const double A = exp(row_dot<LW>(geo, u, bet, ln, mask));
             const double* __restrict__ Es = geo.E + __ldg(sbase + sl);
             const int64_t e0 = __ldg(gp + sl) + jc * CH;
             const int64_t e1 = min(e0 + CH, __ldg(gp + sl + 1));
             // batches of kGrpUnr entries per lane, software-pipelined: the
             // next batch's entries are in flight while this batch gathers
             // exp(offset) and accumulates
-            int64_t e = e0 + lane;
+            int64_t e = e0 + ln;
             constexpr int U8 = kGrpUnr;
-            if (e + 32 * (U8 - 1) < e1) {
+            if (e + LW * (U8 - 1) < e1) {
                 ET c[U8];
 #pragma unroll
-                for (int j = 0; j < U8; ++j) c[j] = gent[e + 32 * j];
+                for (int j = 0; j < U8; ++j) c[j] = gent[e + LW * j];
                 for (;;) {
                     double ev[U8];
 #pragma unroll
                     for (int j = 0; j < U8; ++j) ev[j] = __ldg(Es + Ent::loc(c[j]));
-                    const int64_t en = e + 32 * U8;
-                    const bool more = en + 32 * (U8 - 1) < e1;
+                    const int64_t en = e + LW * U8;
+                    const bool more = en + LW * (U8 - 1) < e1;
                     ET cn[U8];
                     if (more) {
 #pragma unroll
-                        for (int j = 0; j < U8; ++j) cn[j] = gent[en + 32 * j];
+                        for (int j = 0; j < U8; ++j) cn[j] = gent[en + LW * j];
                     }
 #pragma unroll
                     for (int j = 0; j < U8; ++j) Pass::template sparse<double>(gpar, A * ev[j], Ent::y(c[j]), acc);
@@ -821,20 +843,20 @@ __global__ void __launch_bounds__(256) grp_pass_kernel(GrpGeom geo, typename Pas
                     for (int j = 0; j < U8; ++j) c[j] = cn[j];
                 }
             }
-            for (; e < e1; e += 32) {
+            for (; e < e1; e += LW) {
                 const ET c = gent[e];
                 Pass::template sparse<double>(gpar, A * __ldg(Es + Ent::loc(c)), Ent::y(c), acc);
             }
         }
 #pragma unroll
         for (int i = 0; i < NWV; ++i) {
-            const double v = warp_sum(acc.w[i]);
-            if (lane == 0) up[un * NQ + i] = v;
+            const double v = part_sum<LW>(acc.w[i], mask);
+            if (ln == 0) up[un * NQ + i] = v;
         }
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
-            const double v = warp_sum(acc.s[i]);
-            if (lane == 0) up[un * NQ + NWV + i] = v;
+            const double v = part_sum<LW>(acc.s[i], mask);
+            if (ln == 0) up[un * NQ + NWV + i] = v;
         }
     }
     __syncthreads();
@@ -1529,7 +1551,8 @@ static cudaError_t grp_run(const GrpGeom& geo, const PassParamsAny& pa, PassKind
         kern<<<(unsigned)max_slots, 256, smem, st>>>(geo, prm);
         return cudaGetLastError();
     };
-    return val_u16 ? go(grp_pass_kernel<Pass, uint16_t>) : go(grp_pass_kernel<Pass, float>);
+    constexpr int LW = std::is_same_v<Pass, PassSandwich> ? kGrpPartLanes : 32;
+    return val_u16 ? go(grp_pass_kernel<Pass, uint16_t, LW>) : go(grp_pass_kernel<Pass, float, LW>);
 }
 
 cudaError_t launch_grp_pass(PassKind kind, const GrpGeom& geo, const PassParamsAny& prm, int val_u16,
