@@ -570,9 +570,12 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
     } else {
         // software pipeline: the next two cells' rows are in flight while the
         // gene tile works on the current one (one row ahead left most of an L2
-        // round trip exposed)
-        float xn[2][P];
-        float on[2] = {0.f, 0.f};
+        // round trip exposed); with one column, one cell ahead: the second row's
+        // registers would change the blocks per SM, and with them the segments
+        // that the sums are cut into
+        constexpr int D = P == 1 ? 1 : 2;
+        float xn[D][P];
+        float on[D] = {};
         auto load_cell = [&](int c, int s) {
             if (c < c1) {
                 load_row<P, PP>(geo.X, c, xn[s]);
@@ -584,7 +587,7 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
 #pragma unroll
             for (int i = 0; i < P; ++i) x[i] = xn[s][i];
             const float o = on[s] * kLog2e;
-            load_cell(c + 2 * NT, s);
+            load_cell(c + D * NT, s);
             float zz[P * (P + 1) / 2];
 #pragma unroll
             for (int jj = 0; jj < P; ++jj)
@@ -611,12 +614,16 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
         };
         int c = c0 + threadIdx.x;
         load_cell(c, 0);
-        load_cell(c + NT, 1);
-        for (; c + NT < c1; c += 2 * NT) {
-            cell(c, 0);
-            cell(c + NT, 1);
+        if constexpr (D == 1) {
+            for (; c < c1; c += NT) cell(c, 0);
+        } else {
+            load_cell(c + NT, 1);
+            for (; c + NT < c1; c += 2 * NT) {
+                cell(c, 0);
+                cell(c + NT, 1);
+            }
+            if (c < c1) cell(c, 0);
         }
-        if (c < c1) cell(c, 0);
     }
     // sparse corrections: UNR independent nonzeros per thread per step, so
     // their dependent (index -> design row) loads overlap
