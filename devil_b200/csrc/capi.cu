@@ -1272,7 +1272,8 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
                  int nseg, int tiles, const int32_t* bound, const int64_t* segptr,
                  int nbound, const int32_t* act, const int32_t* n_act, int32_t* reset_next,
                  const PassBuffers& pb, const PassParamsAny& prm, int fine = 0,
-                 const int32_t* n_heavy = nullptr, bool rowexp_fresh = false, bool want_vec = true) {
+                 const int32_t* n_heavy = nullptr, bool rowexp_fresh = false, bool want_vec = true,
+                 bool follows = false) {
     if (plan.engine != ENGINE_GRP && !dp.Xrm) fail(ctx, DEVIL_ERR_ARG, "per-cell pass without the per-cell design");
     PassLaunch L;
     L.kind = kind;
@@ -1306,6 +1307,7 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
     L.prm = prm;
     L.stream = ctx->stream;
     L.plain = plan.plain;
+    L.dependent = follows;
     size_t e0 = ctx->profiling ? prof_event(ctx) : 0;
     // (the FP64 matrix engine is, to callers, the per-cell engine of its p)
     ctx->last_engine[kind] = (int)(plan.engine != ENGINE_C64 ? plan.engine
@@ -1567,6 +1569,7 @@ int64_t irls_loop(devil_ctx* ctx, const DevProblem& dp, const PassPlan& plan0, d
     int32_t* cnt = ws<int32_t>(ctx, "cnt", 4);
     LAUNCH(launch_set_i32(cnt, (int32_t)n0, st));
     LAUNCH(launch_set_i32(cnt + 1, 0, st));
+    LAUNCH(launch_set_i32(cnt + 3, 0, st));  // the step's ticket
     PassParamsAny prm{beta_f, beta, k, nullptr, nullptr};
     const PassPlan plan = autotune(ctx, dp, plan0, act[0], cnt, n0, prm, form);
     PassBuffers pb = pass_buffers(ctx, PASS_IRLS, dp.P, max_slot_segs(ctx, dp, plan, form));
@@ -1595,7 +1598,7 @@ int64_t irls_loop(devil_ctx* ctx, const DevProblem& dp, const PassPlan& plan0, d
         // (after the first pass the step kernel keeps the genes' exp(x_u . beta))
         launch_pass(ctx, dp, PASS_IRLS, plan, nseg, tiles, dp.fine_bound, dp.fine_ptr,
                     dp.nfine + 1, act[cur], cnt + cur, cnt + nxt, pb, prm, 0, sliced ? nheavy + cur : nullptr,
-                    sliced && t > 0);
+                    sliced && t > 0, true, t > 0);
         ++launched;
         const bool part_f64 = plan.engine != ENGINE_REG && plan.engine != ENGINE_TC && plan.engine != ENGINE_TCW;
         if (sliced) {
@@ -1615,8 +1618,7 @@ int64_t irls_loop(devil_ctx* ctx, const DevProblem& dp, const PassPlan& plan0, d
         } else {
             LAUNCH(launch_irls_finalize(pb.partW, part_f64, nseg, tiles * plan.GT, dp.P, act[cur],
                                         cnt + cur, (int)hint, act[nxt], cnt + nxt, beta, beta_f,
-                                        iters, status, max_iter, eps, k, st));
-            LAUNCH(launch_copy_i32_to_host_mapped(cnt + nxt, ctx->mapped_dev + (t & 3), st));
+                                        iters, status, max_iter, eps, k, cnt + 3, ctx->mapped_dev + (t & 3), st));
         }
         CK(cudaEventRecord(ctx->ev[t & 3], st));
         if (t >= LAG) CK(cudaEventSynchronize(ctx->ev[(t - LAG) & 3]));
@@ -1741,6 +1743,7 @@ void run_mle(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, const do
     int32_t* cnt = ws<int32_t>(ctx, "cnt", 4);
     LAUNCH(launch_set_i32(cnt, 0, st));
     LAUNCH(launch_set_i32(cnt + 1, 0, st));
+    LAUNCH(launch_set_i32(cnt + 3, 0, st));  // the step's ticket
     // slice-major passes: the active genes stay in decreasing order of entries
     const bool ordered = plan.engine == ENGINE_GRP && (ctx->grp_slices & 2);
     // (and those below kLightEntriesMle entries per slice take eight lanes each)
@@ -1768,7 +1771,7 @@ void run_mle(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, const do
         // (beta is fixed during the MLE loop: exp(x_u . beta) from its first pass)
         launch_pass(ctx, dp, PASS_MLE, plan, nseg, tiles, dp.fine_bound,
                     dp.fine_ptr, dp.nfine + 1, act[cur], cnt + cur, cnt + nxt, pb, prm, 0,
-                    ordered ? nheavy + cur : nullptr, ordered && t > 0);
+                    ordered ? nheavy + cur : nullptr, ordered && t > 0, true, t > 0);
         ++launched;
         const bool part_f64 = plan.engine != ENGINE_REG && plan.engine != ENGINE_TC && plan.engine != ENGINE_TCW;
         // the exclusive-column (one-hot) structure of a grouped design
@@ -1776,14 +1779,13 @@ void run_mle(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, const do
         const bool structured = plan.engine == ENGINE_GRP && dp.grp.nA > 0;
         LAUNCH(launch_mle_finalize(pb.partW, part_f64, pb.partS, nseg, tiles * plan.GT, dp.P, dp.stats, dp.n,
                                    act[cur], cnt + cur, (int)hint, act[nxt], cnt + nxt, s, max_iter,
-                                   cox_reid, nullptr, st, structured ? dp.grp.nA : 0,
+                                   cox_reid, cnt + 3, ordered ? nullptr : ctx->mapped_dev + (t & 3), st,
+                                   structured ? dp.grp.nA : 0,
                                    structured ? dp.grp.colA : nullptr, structured ? dp.grp.colD : nullptr));
-        // (the compaction mirrors the count for the host; otherwise a kernel does)
+        // (the compaction mirrors the count for the host, or the step does)
         if (ordered)
             LAUNCH(launch_compact_kept(act[cur], cnt + cur, 0, s.keep, act[nxt], cnt + nxt, st, dp.grp.wkey, thr,
                                        nheavy + nxt, ctx->mapped_dev + (t & 3)));
-        else
-            LAUNCH(launch_copy_i32_to_host_mapped(cnt + nxt, ctx->mapped_dev + (t & 3), st));
         CK(cudaEventRecord(ctx->ev[t & 3], st));
         if (t >= LAG) CK(cudaEventSynchronize(ctx->ev[(t - LAG) & 3]));
     }

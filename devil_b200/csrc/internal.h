@@ -43,6 +43,7 @@ struct PassLaunch {
     PassParamsAny prm;
     cudaStream_t stream;
     int* occ_out = nullptr;  // non-null: report the kernel's resident blocks per SM, launch nothing
+    int dependent = 0;       // straight after the step of the iteration before (register engine: launch_dependent)
     int plain = 0;           // the plain comparison form (FP32 staging in the shared-memory engine)
     int vec = 1;             // bread pass: the score sums too (clusters); the FP64 matrix engine can leave them out
 };
@@ -57,6 +58,24 @@ size_t gen_smem_bytes(PassKind k, int P, int GT, int plain);
 bool gen_f32_staging(PassKind k, int plain);
 
 cudaError_t launch_reg_pass(const PassLaunch& L);
+
+// launches a kernel that calls grid_wait() first (common.cuh): it may become
+// resident while the kernel before it in the stream still runs
+template <class... KA, class... A>
+cudaError_t launch_dependent(void (*kern)(KA...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                             A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}
 
 // Raise the kernel's dynamic shared-memory cap to at least `bytes` on the
 // current device; never lowers it.  The cap is process-wide per kernel, so
@@ -383,8 +402,6 @@ cudaError_t launch_compact_kept(const int32_t* act, const int32_t* n_act, int64_
                                 volatile int32_t* mirror = nullptr);
 // *out = the number of leading entries of key (in descending order) >= thr
 cudaError_t launch_count_at_least(const int32_t* key, int64_t n, int32_t thr, int32_t* out, cudaStream_t st);
-cudaError_t launch_copy_i32_to_host_mapped(const int32_t* src, volatile int32_t* dst,
-                                           cudaStream_t st);
 
 // ---- finalize kernels (kernels_fin.cu) ----
 // wide: partial sums are FP64 (generic engine) instead of FP32
@@ -392,7 +409,7 @@ cudaError_t launch_irls_finalize(const void* partW, bool wide, int nseg, int slo
                                  const int32_t* act, const int32_t* n_act, int max_slots,
                                  int32_t* act_next, int32_t* n_next, double* beta, float* beta_f,
                                  int32_t* iters, int32_t* status, int max_iter, double eps,
-                                 const float* k, cudaStream_t st);
+                                 const float* k, int32_t* ticket, volatile int32_t* mirror, cudaStream_t st);
 // the IRLS step of the design-group engine's slice-major pass, the p x p
 // assembly from geo.gsum folded in (geo.act / geo.n_act: this iteration's
 // active genes)
@@ -424,7 +441,7 @@ cudaError_t launch_mle_finalize(const void* partW, bool wide, const double* part
                                 int slot_stride, int P, const double* stats, int64_t n,
                                 const int32_t* act, const int32_t* n_act, int max_slots,
                                 int32_t* act_next, int32_t* n_next, MleState s, int max_iter,
-                                int cox_reid, volatile int32_t* mirror, cudaStream_t st, int nA = 0,
+                                int cox_reid, int32_t* ticket, volatile int32_t* mirror, cudaStream_t st, int nA = 0,
                                 const int32_t* colA = nullptr, const int32_t* colD = nullptr);
 cudaError_t launch_sandwich_finalize(const double* partW, int nseg, int slot_stride, int P,
                                      const int32_t* seg_cluster, int n_clusters, int64_t n,

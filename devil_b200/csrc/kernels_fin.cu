@@ -29,7 +29,7 @@ DEV void reduce_partials(const T* part, int nseg, int slot_stride, int slot, int
             for (int u = 0; u < U; ++u)
 #pragma unroll
                 for (int j = 0; j < A; ++j)
-                    v[j][u] = s0 + u < nseg && a0 + 32 * j < count ? __ldg(p + u * step + 32 * j) : T(0);
+                    v[j][u] = s0 + u < nseg && a0 + 32 * j < count ? p[u * step + 32 * j] : T(0);
 #pragma unroll
             for (int j = 0; j < A; ++j)
 #pragma unroll
@@ -62,7 +62,7 @@ DEV void unpack_sym(int P, const double* packed, double* M) {
 // converged when max|delta| < eps; NaN in delta[0] stops the gene.
 // ------------------------------------------------------------------
 template <class TW>
-__global__ void irls_finalize_kernel(const TW* partW, int nseg, int slot_stride, int P,
+DEV void irls_finalize_gene(const TW* partW, int nseg, int slot_stride, int P,
                                      const int32_t* act, const int32_t* n_act, int32_t* act_next,
                                      int32_t* n_next, double* beta, float* beta_f, int32_t* iters,
                                      int32_t* status, int max_iter, double eps, const float* kf) {
@@ -114,11 +114,39 @@ __global__ void irls_finalize_kernel(const TW* partW, int nseg, int slot_stride,
     }
 }
 
+// The block that ends last tells the host how many genes go on (mirror: its
+// pinned, mapped copy; ticket: the blocks that have ended, 0 between launches).
+// As a kernel of its own this took 3 us of each iteration, and a launch.
+DEV void mirror_by_last_block(const int32_t* n_next, int32_t* ticket, volatile int32_t* mirror) {
+    if (!mirror) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(ticket, 1) != (int)gridDim.x - 1) return;
+    *ticket = 0;
+    __threadfence();
+    *mirror = *(const volatile int32_t*)n_next;
+}
+
+template <class TW>
+__global__ void irls_finalize_kernel(const TW* partW, int nseg, int slot_stride, int P,
+                                     const int32_t* act, const int32_t* n_act, int32_t* act_next,
+                                     int32_t* n_next, double* beta, float* beta_f, int32_t* iters,
+                                     int32_t* status, int max_iter, double eps, const float* kf,
+                                     int32_t* ticket, volatile int32_t* mirror) {
+    grid_trigger();
+    grid_wait();
+    irls_finalize_gene(partW, nseg, slot_stride, P, act, n_act, act_next, n_next, beta, beta_f, iters, status,
+                       max_iter, eps, kf);
+    mirror_by_last_block(n_next, ticket, mirror);
+}
+
 cudaError_t launch_irls_finalize(const void* partW, bool wide, int nseg, int slot_stride, int P,
                                  const int32_t* act, const int32_t* n_act, int max_slots,
                                  int32_t* act_next, int32_t* n_next, double* beta, float* beta_f,
                                  int32_t* iters, int32_t* status, int max_iter, double eps,
-                                 const float* k, cudaStream_t st) {
+                                 const float* k, int32_t* ticket, volatile int32_t* mirror,
+                                 cudaStream_t st) {
     if (max_slots <= 0) return cudaSuccess;
     const int NA = P * (P + 1) / 2 + P;
     const size_t per = (size_t)(NA + P * wla_ld(P) + P) * sizeof(double);
@@ -130,10 +158,9 @@ cudaError_t launch_irls_finalize(const void* partW, bool wide, int nseg, int slo
             cudaError_t e = raise_dyn_smem(irls_finalize_kernel<TW>, smem);
             if (e != cudaSuccess) return e;
         }
-        irls_finalize_kernel<TW><<<nblk(max_slots, w), 32 * w, smem, st>>>(
-            pw, nseg, slot_stride, P, act, n_act, act_next, n_next, beta, beta_f, iters, status,
-            max_iter, eps, k);
-        return cudaGetLastError();
+        return launch_dependent(irls_finalize_kernel<TW>, nblk(max_slots, w), 32 * w, smem, st, pw, nseg,
+                                slot_stride, P, act, n_act, act_next, n_next, beta, beta_f, iters, status, max_iter,
+                                eps, k, ticket, mirror);
     };
     // the register engine leaves FP32 partial sums, the generic engine FP64
     return wide ? go(static_cast<const double*>(partW)) : go(static_cast<const float*>(partW));
@@ -210,6 +237,8 @@ __global__ void grp_irls_finalize_kernel(GrpGeom geo, int32_t* act_next, int32_t
                                          int32_t* status, int max_iter, double eps,
                                          const float* kf, int8_t* keep) {
     extern __shared__ double fsh[];
+    grid_trigger();
+    grid_wait();
     const int P = geo.P, U = geo.U, S = geo.S, LD = wla_ld(P);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // group sums, then H (P x LD) for the LU step, or the compact store of
@@ -360,9 +389,8 @@ cudaError_t launch_grp_irls_finalize(const GrpGeom& geo, int max_slots, int32_t*
         cudaError_t e = raise_dyn_smem(grp_irls_finalize_kernel, smem);
         if (e != cudaSuccess) return e;
     }
-    grp_irls_finalize_kernel<<<nblk(max_slots, w), 32 * w, smem, st>>>(
-        geo, act_next, n_next, beta, beta_f, iters, status, max_iter, eps, k, keep);
-    return cudaGetLastError();
+    return launch_dependent(grp_irls_finalize_kernel, nblk(max_slots, w), 32 * w, smem, st, geo, act_next, n_next, beta,
+                            beta_f, iters, status, max_iter, eps, k, keep);
 }
 
 // ------------------------------------------------------------------
@@ -552,7 +580,7 @@ DEV void mle_cr_structured(const double* sums, int P, int NE, int k, const int32
 }
 
 template <class TW>
-__global__ void mle_finalize_kernel(const TW* partW, const double* partS, int nseg,
+DEV void mle_finalize_gene(const TW* partW, const double* partS, int nseg,
                                     int slot_stride, int P, const double* stats, int64_t n,
                                     const int32_t* act, const int32_t* n_act, int32_t* act_next,
                                     int32_t* n_next, MleState st, int max_iter, int cox_reid,
@@ -696,13 +724,25 @@ __global__ void mle_finalize_kernel(const TW* partW, const double* partS, int ns
     }
     if (st.keep) st.keep[g] = done ? 0 : 1;
 }
+template <class TW>
+__global__ void mle_finalize_kernel(const TW* partW, const double* partS, int nseg,
+                                    int slot_stride, int P, const double* stats, int64_t n,
+                                    const int32_t* act, const int32_t* n_act, int32_t* act_next,
+                                    int32_t* n_next, MleState st, int max_iter, int cox_reid,
+                                    int nA, const int32_t* colA, const int32_t* colD, int32_t* ticket,
+                                    volatile int32_t* mirror) {
+    grid_trigger();
+    grid_wait();
+    mle_finalize_gene(partW, partS, nseg, slot_stride, P, stats, n, act, n_act, act_next, n_next, st, max_iter,
+                      cox_reid, nA, colA, colD);
+    mirror_by_last_block(n_next, ticket, mirror);
+}
 cudaError_t launch_mle_finalize(const void* partW, bool wide, const double* partS, int nseg,
                                 int slot_stride, int P, const double* stats, int64_t n,
                                 const int32_t* act, const int32_t* n_act, int max_slots,
                                 int32_t* act_next, int32_t* n_next, MleState s, int max_iter,
-                                int cox_reid, volatile int32_t* mirror, cudaStream_t st, int nA,
+                                int cox_reid, int32_t* ticket, volatile int32_t* mirror, cudaStream_t st, int nA,
                                 const int32_t* colA, const int32_t* colD) {
-    (void)mirror;
     if (max_slots <= 0) return cudaSuccess;
     const int NA = 3 * (P * (P + 1) / 2) + 2;
     const size_t per = (size_t)(NA + 6 + (nA > 0 ? 6 * nA * nA : 4 * P * wla_ld(P)) + P) * sizeof(double);
@@ -714,10 +754,9 @@ cudaError_t launch_mle_finalize(const void* partW, bool wide, const double* part
             cudaError_t e = raise_dyn_smem(mle_finalize_kernel<TW>, smem);
             if (e != cudaSuccess) return e;
         }
-        mle_finalize_kernel<TW><<<nblk(max_slots, w), 32 * w, smem, st>>>(
-            pw, partS, nseg, slot_stride, P, stats, n, act, n_act, act_next, n_next, s, max_iter,
-            cox_reid, nA, colA, colD);
-        return cudaGetLastError();
+        return launch_dependent(mle_finalize_kernel<TW>, nblk(max_slots, w), 32 * w, smem, st, pw, partS, nseg,
+                                slot_stride, P, stats, n, act, n_act, act_next, n_next, s, max_iter, cox_reid, nA, colA,
+                                colD, ticket, mirror);
     };
     return wide ? go(static_cast<const double*>(partW)) : go(static_cast<const float*>(partW));
 }

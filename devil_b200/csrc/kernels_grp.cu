@@ -972,17 +972,8 @@ __global__ void __launch_bounds__(kSlNT, 1) grp_slices_kernel(GrpGeom geo, typen
     constexpr int EPL = sizeof(uint4) / sizeof(ET);  // entries per 16-byte piece
     constexpr int UNR = sl_unr<Pass>();
     constexpr int RW = 32 * UNR;                      // 16-byte pieces per round
-    if (geo.reset_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *geo.reset_next = 0;
+    grid_trigger();
     (void)tile;
-    const int nact = *geo.n_act;
-    // genes [0, nheavy) of the list take a warp each, the rest eight lanes each
-    const int nheavy = geo.n_heavy ? min(nact, *geo.n_heavy) : nact;
-    // block y takes the slots y, y + T, y + 2T, ... (T = gridDim.y) of each
-    // part: with the active genes listed in decreasing order of entries,
-    // every block gets a like share of the work and hands its largest genes
-    // out first, so the block's last warps finish together
-    const int T = gridDim.y, y = blockIdx.y;
-    if (y >= nact) return;
     const int s = blockIdx.x, S = geo.S, U = geo.U;
     extern __shared__ double Es[];  // [kSliceCells] exp(offset) of the slice's cells
     const int c0 = __ldg(geo.sl_start + s), nc = __ldg(geo.sl_start + s + 1) - c0;
@@ -1020,6 +1011,19 @@ __global__ void __launch_bounds__(kSlNT, 1) grp_slices_kernel(GrpGeom geo, typen
         rule[j] = __ldg(geo.rw + (int64_t)u * kRuleCap + j);
         rule[kRuleCap + j] = __ldg(geo.res + (int64_t)u * kRuleCap + j);
     }
+    // what the step before this pass writes is read from here on (the slice and
+    // its rule are staged while that step still runs)
+    grid_wait();
+    if (geo.reset_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *geo.reset_next = 0;
+    const int nact = *geo.n_act;
+    // genes [0, nheavy) of the list take a warp each, the rest eight lanes each
+    const int nheavy = geo.n_heavy ? min(nact, *geo.n_heavy) : nact;
+    // block y takes the slots y, y + T, y + 2T, ... (T = gridDim.y) of each
+    // part: with the active genes listed in decreasing order of entries,
+    // every block gets a like share of the work and hands its largest genes
+    // out first, so the block's last warps finish together
+    const int T = gridDim.y, y = blockIdx.y;
+    if (y >= nact) return;
     const uint4* __restrict__ v4 = static_cast<const uint4*>(geo.gent);
     // the block's genes are handed out one at a time (a shared counter), so
     // warps that drew short genes take more of them
@@ -1035,8 +1039,8 @@ __global__ void __launch_bounds__(kSlNT, 1) grp_slices_kernel(GrpGeom geo, typen
         SlItem it{y + __shfl_sync(0xffffffffu, k, 0) * T, 0, 0.0, 0, 0};
         if (it.j >= nheavy) it.j = nact;  // past the heavy part
         if (it.j < nact) {
-            it.g = __ldg(geo.act + it.j);
-            it.A = __ldg(geo.rowexp + (int64_t)it.g * U + u);
+            it.g = __ldcg(geo.act + it.j);
+            it.A = __ldcg(geo.rowexp + (int64_t)it.g * U + u);
             it.e0 = __ldg(geo.gptr + (int64_t)it.g * (S + 1) + s);
             it.e1 = __ldg(geo.gptr + (int64_t)it.g * (S + 1) + s + 1);
         }
@@ -1220,8 +1224,8 @@ __global__ void __launch_bounds__(kSlNT, 1) grp_slices_kernel(GrpGeom geo, typen
             const int jl = y + (k0 + sub) * T;
             SlItem it{jl < nlight ? nheavy + jl : -1, 0, 0.0, 0, 0};
             if (it.j >= 0) {
-                it.g = __ldg(geo.act + it.j);
-                it.A = __ldg(geo.rowexp + (int64_t)it.g * U + u);
+                it.g = __ldcg(geo.act + it.j);
+                it.A = __ldcg(geo.rowexp + (int64_t)it.g * U + u);
                 it.e0 = __ldg(geo.gptr + (int64_t)it.g * (S + 1) + s);
                 it.e1 = __ldg(geo.gptr + (int64_t)it.g * (S + 1) + s + 1);
             }
@@ -1440,6 +1444,8 @@ static cudaError_t slices_run(const GrpGeom& geo, typename Pass::Params prm, int
     auto go = [&](auto kern) -> cudaError_t {
         cudaError_t e = raise_dyn_smem(kern, smem);
         if (e != cudaSuccess) return e;
+        // straight after the step of the iteration before: see grid_wait
+        if (rowexp_fresh && !Pass::TABLES) return launch_dependent(kern, grid, kSlNT, smem, st, geo, prm, tile);
         kern<<<grid, kSlNT, smem, st>>>(geo, prm, tile);
         return cudaGetLastError();
     };

@@ -1171,6 +1171,8 @@ __global__ void __launch_bounds__(kCompactNT) compact_kept_kernel(const int32_t*
                                                                   volatile int32_t* mirror) {
     __shared__ int wtot[kCompactR][32];
     __shared__ int batch_total;
+    grid_trigger();
+    grid_wait();
     const int64_t n = n_act ? (int64_t)*n_act : n_fixed;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -1238,9 +1240,8 @@ __global__ void __launch_bounds__(kCompactNT) compact_kept_kernel(const int32_t*
 cudaError_t launch_compact_kept(const int32_t* act, const int32_t* n_act, int64_t n_fixed, const int8_t* keep,
                                 int32_t* act_next, int32_t* n_next, cudaStream_t st, const int32_t* wkey,
                                 int32_t thr, int32_t* n_heavy_next, volatile int32_t* mirror) {
-    compact_kept_kernel<<<1, kCompactNT, 0, st>>>(act, n_act, n_fixed, keep, act_next, n_next, wkey, thr,
-                                                  n_heavy_next, mirror);
-    return cudaGetLastError();
+    return launch_dependent(compact_kept_kernel, 1, kCompactNT, 0, st, act, n_act, n_fixed, keep, act_next, n_next, wkey,
+                            thr, n_heavy_next, mirror);
 }
 // *out = the number of leading entries of key (descending) that are >= thr
 __global__ void count_at_least_kernel(const int32_t* key, int64_t n, int32_t thr, int32_t* out) {
@@ -1260,11 +1261,4 @@ cudaError_t launch_set_i32(int32_t* a, int32_t v, cudaStream_t st) {
     set_i32_kernel<<<1, 1, 0, st>>>(a, v);
     return cudaGetLastError();
 }
-__global__ void mirror_kernel(const int32_t* src, volatile int32_t* dst) { *dst = *src; }
-cudaError_t launch_copy_i32_to_host_mapped(const int32_t* src, volatile int32_t* dst,
-                                           cudaStream_t st) {
-    mirror_kernel<<<1, 1, 0, st>>>(src, dst);
-    return cudaGetLastError();
-}
-
 }  // namespace devil

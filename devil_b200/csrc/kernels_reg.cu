@@ -77,18 +77,17 @@ static cudaError_t run(const PassLaunch& L) {
             return cudaGetLastError();
         }
     }
-    if constexpr (K == PASS_IRLS) {
-        if (L.val_u16)
-            reg_pass_kernel<P, PP, GT, kRegNT, Pass, uint16_t><<<grid, kRegNT, 0, L.stream>>>(L.geo, prm);
-        else
-            reg_pass_kernel<P, PP, GT, kRegNT, Pass, float><<<grid, kRegNT, 0, L.stream>>>(L.geo, prm);
-    } else {
-        if (L.val_u16)
-            reg_pass_kernel_b1<P, PP, GT, kRegNT, Pass, uint16_t><<<grid, kRegNT, 0, L.stream>>>(L.geo, prm);
-        else
-            reg_pass_kernel_b1<P, PP, GT, kRegNT, Pass, float><<<grid, kRegNT, 0, L.stream>>>(L.geo, prm);
-    }
-    return cudaGetLastError();
+    auto go = [&](auto k) -> cudaError_t {
+        if (L.dependent) return launch_dependent(k, grid, kRegNT, 0, L.stream, L.geo, prm);
+        k<<<grid, kRegNT, 0, L.stream>>>(L.geo, prm);
+        return cudaGetLastError();
+    };
+    if constexpr (K == PASS_IRLS)
+        return L.val_u16 ? go(reg_pass_kernel<P, PP, GT, kRegNT, Pass, uint16_t>)
+                         : go(reg_pass_kernel<P, PP, GT, kRegNT, Pass, float>);
+    else
+        return L.val_u16 ? go(reg_pass_kernel_b1<P, PP, GT, kRegNT, Pass, uint16_t>)
+                         : go(reg_pass_kernel_b1<P, PP, GT, kRegNT, Pass, float>);
 }
 
 template <PassKind K, int P>

@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
     __shared__ int16_t ptab[kWNmax];  // product row -> i | j << 8 (-1: padding)
     __shared__ double psia[MLE ? kMleG : 1];
 
+    grid_trigger();
     if (geo.reset_next && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0)
         *geo.reset_next = 0;
     const int nact = *geo.n_act;

@@ -484,6 +484,8 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
     using AW = typename Pass::AW;
     using AS = typename Pass::AS;
 
+    grid_trigger();
+    grid_wait();
     if (geo.reset_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *geo.reset_next = 0;
     const int nact = *geo.n_act;
     const int tile = blockIdx.y;
@@ -500,14 +502,14 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
     for (int j = 0; j < GT; ++j) {
         int slot = tile * GT + j;
         if (slot >= nact) slot = tile * GT;  // duplicate a valid gene; not written
-        int g = __ldg(geo.act + slot);
+        int g = __ldcg(geo.act + slot);
         gid[j] = g;
         if constexpr (F64) {
 #pragma unroll
-            for (int i = 0; i < P; ++i) betad[j][i] = __ldg(prm.beta_d + (int64_t)g * P + i);
+            for (int i = 0; i < P; ++i) betad[j][i] = __ldcg(prm.beta_d + (int64_t)g * P + i);
         } else {
 #pragma unroll
-            for (int i = 0; i < P; ++i) beta[j][i] = __ldg(prm.beta + (int64_t)g * P + i) * kLog2e;
+            for (int i = 0; i < P; ++i) beta[j][i] = __ldcg(prm.beta + (int64_t)g * P + i) * kLog2e;
         }
         gp[j] = Pass::load(prm, g);
     }
