@@ -2164,14 +2164,14 @@ void read_settings(devil_ctx* ctx) {
     ctx->debug = (dbg && atoi(dbg)) ? 1 : 0;
 }
 // The workers' contexts after a batch: kept for the next one while their
-// workspaces hold less than 1/32 of the device, until the context ends or runs
+// workspaces hold less than 1/64 of the device, until the context ends or runs
 // out of memory; destroyed after an error, or when another call's are kept.
 void keep_batch(devil_ctx* ctx, std::vector<devil_ctx*>& wc, bool ok) {
     size_t held = 0, free_b = 0, total = 0;
     for (auto* c : wc)
         for (auto& kv : c->bufs) held += kv.second.bytes;
     if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) ok = false;
-    if (ok && held <= total / 32) {
+    if (ok && held <= total / 64) {
         std::lock_guard<std::mutex> lk(ctx->batch_mu);
         if (ctx->batch.empty()) ctx->batch.swap(wc);
     }
