@@ -696,6 +696,17 @@ void compute_offsets(devil_ctx* ctx, DevProblem& dp, int method, const double* s
              "Please filter out empty samples from input matrix.");
 }
 
+// The searches for theta amplify rounding, so the sums of beta before them keep
+// one order, whatever the clusters and group sizes, and a data set's fit repeats
+// from build to build.  The MLE's Newton search resolves its last bracket at
+// rounding level: beta moved by 1e-15 moves theta by up to 1e-7 on a few genes in
+// 10,000.  The "new" search is ill-conditioned on near-Poisson genes: beta moved
+// by 1e-13 (two conditions, 150,000 cells) moved theta by up to 2.4 %, and by more
+// than 1e-9 on half of 111 genes.
+bool search_follows(int overdispersion) {
+    return overdispersion == DEVIL_OD_MLE || overdispersion == DEVIL_OD_NEW;
+}
+
 // ------------------------------------------------------------------
 // design groups: distinct design rows (x cluster) of the cells, their
 // Gauss rules and the CSR copy ordered by group (kernels_grp.cu).  Used
@@ -819,14 +830,12 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     // walks the pieces (slice x cluster): within a design row the cells are in
     // cluster order, so a gene's entries of a slice are too, and a piece is a
     // run of them (f_ptr).
-    // A fit with the MLE dispersion cuts at the clusters too.  Its Newton search
-    // resolves the last bracket at rounding level, so sums in another order move
-    // theta by up to 1e-7 on a few genes in 10,000 (beta by 1e-15): fits of one
-    // data set would no longer repeat those of earlier builds to 1e-9.
+    // Where a search for the dispersion follows (search_follows) the slices are
+    // cut at the clusters too, so that the order of every sum stays.
     std::vector<int64_t> hks(K + 1);
     CK(cudaMemcpyAsync(hks.data(), kst, (K + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    const bool by_cluster = overdispersion == DEVIL_OD_MLE;
+    const bool by_cluster = search_follows(overdispersion);
     std::vector<int32_t> sl_start{0}, sl_key, kslice(U + 1);
     std::vector<int32_t> f_key, f_base, f_slice, f_loc, f_kslice(K + 1);
     for (int u = 0; u < U; ++u) {
@@ -879,8 +888,8 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     int32_t* rm = ws<int32_t>(ctx, "grp_rm", nrules);
     double* scr = ws<double>(ctx, "grp_scr", (size_t)4 * n);
     double* rerr = ws<double>(ctx, "grp_rerr", nrules);
-    // (MLE: the rules' sums in one order whatever the group sizes, as for the slices)
-    const bool one_block = overdispersion == DEVIL_OD_MLE;
+    // (a search: the rules' sums in one order whatever the group sizes, as for the slices)
+    const bool one_block = search_follows(overdispersion);
     LAUNCH(launch_group_rules(permC, gsC, U, dp.off, n, scr, rs, rw, rm, rerr, bad + 1, one_block, st));
     if (C > 1)  // rules U.. : the (row, cluster) groups
         LAUNCH(launch_group_rules(permF, gsF, K, dp.off, n, scr, rs + (size_t)U * kRuleCap,
@@ -2565,8 +2574,9 @@ int devil_beta_fit(devil_ctx* ctx, const devil_counts* counts, const double* X, 
         upload_counts(ctx, counts, dp);
         prepare_design(ctx, dp, X, p, false);
         upload_offsets(ctx, dp, offset_vector);
-        build_groups(ctx, dp, nullptr, 0, form, DEVIL_OD_NONE);
-        cells_if_needed(ctx, dp, 0, DEVIL_OD_NONE);
+        // (the caller may search for theta at these coefficients)
+        build_groups(ctx, dp, nullptr, 0, form, DEVIL_OD_MLE);
+        cells_if_needed(ctx, dp, 0, DEVIL_OD_MLE);
         const int64_t G = dp.G;
         double* b = ws<double>(ctx, "beta", (size_t)G * p);
         float* bf = ws<float>(ctx, "beta_f", (size_t)G * p);
