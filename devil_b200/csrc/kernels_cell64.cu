@@ -3,11 +3,12 @@
 // :207-217; PassSandwich of passes.cuh) and MOM moments
 // (src/mom_overdispersion.cpp:34-45; PassMOM, mom_cells_kernel below).
 //
-// Bread, per gene and cell: eta = off + x . beta, mu = exp(eta), the weight; then sum_c w_gc x_ci x_cj for every i <= j: a contraction of the weights
-// (genes x cells) with the products z (cells x p (p + 1) / 2).  Both run on the
-// FP64 matrix instruction (mma.m8n8k4): eta of 8 genes x 8 cells, and 16 genes x
-// 8 products per warp and step, so an operand element is fetched once per 8 or
-// 16 multiply-adds instead of once per two.
+// Bread, per gene and cell: eta = off + x . beta, mu = exp(eta), the weight; then
+// sum_c w_gc x_ci x_cj for every i <= j: a contraction of the weights (genes x
+// cells) with the products z (cells x p (p + 1) / 2).  Both run on the FP64
+// matrix instruction (mma.m8n8k4): eta of 8 genes x 8 cells, and 16 genes x 8
+// products per warp and step, so an operand element is fetched once per 8 or 16
+// multiply-adds instead of once per two.
 //
 // Block = 32 genes x one run of cells, 256 threads, chunks of 32 cells: the
 // chunk's design rows by cp.async one chunk ahead, the genes' nonzero counts
@@ -18,6 +19,22 @@
 // 17).  The products are formed at the fetch (two reads and one multiply for two
 // instructions).  Row strides are 4 mod 16 doubles, so the 4 x 4 doubles that
 // half a warp fetches lie in different banks.
+//
+// The accumulators hold the sums of kCRun chunks (64 cells), which are then added
+// to the thread's totals in shared memory: one sum over a whole run of 1,024
+// cells rounds two to ten times as much as short sums of sums do.  Against 80-bit
+// sums, rms of the diagonal scale, 16 genes: p = 9, 2,000 cells 3.5e-16 with one
+// sum, 0.8e-16 so (the shared-memory engine: 0.8e-16); p = 16, 20,000 cells
+// 1.1e-16, 0.6e-16 (0.8e-16); p = 4, 1,500 cells 9.8e-16, 1.1e-16 (the register
+// engine: 1.2e-16).  It costs 500 genes x 20,000 cells 298 -> 306 us at p = 16,
+// 574 -> 588 at p = 24, 929 -> 990 at p = 32.  Two chunks: the error of a run of r
+// cells in s is about u sqrt((r / 3) (r / s) + (s / r) / 3), least at r = 64 to 80
+// for s = 1,024; up to three units (p <= 12) the shared memory takes a second
+// level, four runs to a total, as short as the register engine's sums.
+//
+// Up to nine units a thread keeps to 128 registers for two blocks per SM.  At p =
+// 18..22 it then spills about 88 bytes; with one block and no spill, 4,000 x
+// 50,000, p = 18 takes 5.5 ms instead of 4.8.
 //
 // Bound by the FP64 pipe: exp and the terms, about 45 operations a gene-cell,
 // and p (p + 1) / 2 multiply-adds.  The engine it replaces kept one output per
@@ -37,14 +54,24 @@ constexpr int kCC = 32;   // cells per chunk
 constexpr int kCNT = 256;
 constexpr int kCW = kCG + 4;  // weight row stride (4 mod 16)
 constexpr int kCY = kCC + 1;  // count row stride
+constexpr int kCRun = 2;      // chunks whose sums the accumulators hold (see above)
+constexpr int kCRuns = 4;     // runs in a total where there are two levels of them
 
 // smallest stride >= xs that is 4 mod 16
 __host__ __device__ constexpr int c64_stride(int xs) { return xs + ((20 - xs % 16) % 16); }
 
+// tiles of 8 products (and of 8 score sums), and the units of a warp
+__host__ __device__ constexpr int c64_tiles(int P, bool vec) { return (P * (P + 1) / 2 + 7) / 8 + (vec ? (P + 7) / 8 : 0); }
+__host__ __device__ constexpr int c64_units(int P, bool vec) { return (c64_tiles(P, vec) + 3) / 4; }
+// levels of totals: one per run, and up to three units a second one per kCRuns runs
+__host__ __device__ constexpr int c64_totals(int units) { return units <= 3 ? 2 : 1; }
+
 template <bool VEC>
-__host__ __device__ constexpr size_t c64_smem(int xs) {
+constexpr size_t c64_smem(int P, int xs) {
     return (size_t)(2 * kCC + kCG) * c64_stride(xs) * sizeof(double) +
-           (VEC ? 2 : 1) * (size_t)kCC * kCW * sizeof(double) + (size_t)2 * kCG * kCY * sizeof(float);
+           (VEC ? 2 : 1) * (size_t)kCC * kCW * sizeof(double) +
+           (size_t)c64_totals(c64_units(P, VEC)) * c64_units(P, VEC) * 4 * kCNT * sizeof(double) +
+           (size_t)2 * kCG * kCY * sizeof(float);
 }
 
 // C (8 x 8) += A (8 x 4, row) B (4 x 8, column): lane l holds A[l / 4][l % 4],
@@ -69,7 +96,10 @@ __global__ void __launch_bounds__(kCNT, UN <= 9 ? 2 : 1) cell64_kernel(PassGeom 
     double* xsm = c64sm;                      // [2][kCC][RS] design rows
     double* bsm = xsm + 2 * kCC * RS;         // [kCG][RS] coefficients
     double* wsm = bsm + kCG * RS;             // [VEC ? 2 : 1][kCC][kCW] weights
-    float* ysm = reinterpret_cast<float*>(wsm + (VEC ? 2 : 1) * kCC * kCW);  // [2][kCG][kCY]
+    constexpr int TL = c64_totals(UN);
+    const int TS = c64_units(P, VEC) * 4 * kCNT;
+    double* tot = wsm + (VEC ? 2 : 1) * kCC * kCW;            // [TL][units][4][kCNT] sums of the runs before
+    float* ysm = reinterpret_cast<float*>(tot + TL * TS);     // [2][kCG][kCY]
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, r4 = lane >> 2, k4 = lane & 3;
     const int NE = P * (P + 1) / 2;
 
@@ -166,6 +196,25 @@ __global__ void __launch_bounds__(kCNT, UN <= 9 ? 2 : 1) cell64_kernel(PassGeom 
         }
     }
 
+    // run r's sums into the totals (each thread its own place)
+    auto add_run = [&](int r) {
+        const bool fresh = TL == 2 ? r % kCRuns == 0 : r == 0;
+#pragma unroll
+        for (int i = 0; i < UN; ++i) {
+            if ((warp + 8 * i) >> 1 >= NT) break;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    double& o = tot[(4 * i + 2 * m + q) * kCNT + t];
+                    const double v = fresh ? acc[i][m][q] : o + acc[i][m][q];
+                    acc[i][m][q] = 0.0;
+                    o = v;
+                    if (TL == 2 && r % kCRuns == kCRuns - 1) (&o)[TS] = r < kCRuns ? v : (&o)[TS] + v;
+                }
+        }
+    };
+
     if (nchunk > 0) {
         fetch(c0, 0);
         load_entries();
@@ -176,6 +225,7 @@ __global__ void __launch_bounds__(kCNT, UN <= 9 ? 2 : 1) cell64_kernel(PassGeom 
     for (int k = 0; k < nchunk; ++k) {
         const int cb = c0 + k * kCC, s = k & 1;
         float* ys = ysm + s * kCG * kCY;
+        if (k > 0 && k % kCRun == 0) add_run(k / kCRun - 1);
         scatter(cb, ys);
         load_entries();  // the next chunk's
         cp_async_wait<0>();
@@ -242,8 +292,12 @@ __global__ void __launch_bounds__(kCNT, UN <= 9 ? 2 : 1) cell64_kernel(PassGeom 
         }
     }
     cp_async_wait<0>();
+    const int runs = nchunk > 0 ? (nchunk - 1) / kCRun + 1 : 1;
+    add_run(runs - 1);
     {
         const int NA = NE + P;
+        // the totals: the second level, and runs that did not fill one
+        const bool low = TL == 1 || runs % kCRuns != 0, high = TL == 2 && runs >= kCRuns;
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
             const int nt = (warp + 8 * i) >> 1;
@@ -257,7 +311,8 @@ __global__ void __launch_bounds__(kCNT, UN <= 9 ? 2 : 1) cell64_kernel(PassGeom 
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int n = 8 * (vec ? nt - NTo : nt) + 2 * k4 + q;
-                    if (n < (vec ? P : NE)) o[(vec ? NE : 0) + n] = acc[i][m][q];
+                    const double* v = tot + (4 * i + 2 * m + q) * kCNT + t;
+                    if (n < (vec ? P : NE)) o[(vec ? NE : 0) + n] = (high ? v[TS] : 0.0) + (low ? v[0] : 0.0);
                 }
             }
         }
@@ -448,7 +503,7 @@ cudaError_t run_mom(const PassLaunch& L, int max_slots) {
 
 template <int UN, bool VEC>
 cudaError_t run(const PassLaunch& L) {
-    const size_t smem = c64_smem<VEC>(L.xs_pad);
+    const size_t smem = c64_smem<VEC>(L.P, L.xs_pad);
     auto go = [&](auto kern) -> cudaError_t {
         cudaError_t e = raise_dyn_smem(kern, smem);
         if (e != cudaSuccess) return e;
@@ -461,11 +516,11 @@ cudaError_t run(const PassLaunch& L) {
 
 template <bool VEC>
 cudaError_t run_bread(const PassLaunch& L) {
-    const int NT = (L.P * (L.P + 1) / 2 + 7) / 8 + (VEC ? (L.P + 7) / 8 : 0);
-    if (NT <= 12) return run<3, VEC>(L);
-    if (NT <= 20) return run<5, VEC>(L);
-    if (NT <= 36) return run<9, VEC>(L);
-    if (NT <= 52) return run<13, VEC>(L);
+    const int units = c64_units(L.P, VEC);
+    if (units <= 3) return run<3, VEC>(L);
+    if (units <= 5) return run<5, VEC>(L);
+    if (units <= 9) return run<9, VEC>(L);
+    if (units <= 13) return run<13, VEC>(L);
     return run<18, VEC>(L);
 }
 

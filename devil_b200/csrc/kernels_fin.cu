@@ -12,8 +12,10 @@ static inline unsigned nblk(int64_t m, int t) { return (unsigned)((m + t - 1) / 
 // sums[a] = sum over segments of part[seg][slot][a], in segment order (lanes
 // split a).  Eight segments of two outputs are loaded before they are added: the
 // last genes of a loop leave up to 300 segments, and one load per addition made
-// the step 75 us whatever the number of genes.
-template <class T>
+// the step 75 us whatever the number of genes.  TREE: each eight are summed
+// pairwise first (bread and meat, which no search follows and where a chain over
+// many short segments would round more than the segments do).
+template <bool TREE = false, class T>
 DEV void reduce_partials(const T* part, int nseg, int slot_stride, int slot, int stride, int count,
                          double* sums, int lane) {
     constexpr int A = 2, U = 8;
@@ -30,11 +32,22 @@ DEV void reduce_partials(const T* part, int nseg, int slot_stride, int slot, int
 #pragma unroll
                 for (int j = 0; j < A; ++j)
                     v[j][u] = s0 + u < nseg && a0 + 32 * j < count ? p[u * step + 32 * j] : T(0);
+            if constexpr (TREE) {
 #pragma unroll
-            for (int j = 0; j < A; ++j)
+                for (int h = 1; h < U; h *= 2)
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (s0 + u < nseg) s[j] += (double)v[j][u];
+                    for (int j = 0; j < A; ++j)
+#pragma unroll
+                        for (int u = 0; u < U; u += 2 * h) v[j][u] += v[j][u + h];
+#pragma unroll
+                for (int j = 0; j < A; ++j) s[j] += (double)v[j][0];
+            } else {
+#pragma unroll
+                for (int j = 0; j < A; ++j)
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (s0 + u < nseg) s[j] += (double)v[j][u];
+            }
         }
 #pragma unroll
         for (int j = 0; j < A; ++j)
@@ -785,7 +798,7 @@ __global__ void sandwich_finalize_kernel(const double* partW, int nseg, int slot
     const int slot = blockIdx.x * (blockDim.x >> 5) + warp;
     if (slot >= *n_act) return;
     const int g = act[slot];
-    reduce_partials(partW, nseg, slot_stride, slot, NA, NE, sums, lane);  // H part only
+    reduce_partials<true>(partW, nseg, slot_stride, slot, NA, NE, sums, lane);  // H part only
     for (int i = lane; i < P * LD; i += 32) Mt[i] = 0.0;
     __syncwarp();
     if (n_clusters > 0) {
