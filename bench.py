@@ -448,6 +448,7 @@ def time_plain(args, L, lib, ctx, dev, ext, data, X, p, n, sf_dev, opts_chosen, 
            "value": k / (ms_plain / 1e3), "unit": "genes/s",
            "chosen_same_sample": {"ms_per_step": ms_chosen, "value": k / (ms_chosen / 1e3)},
            "engines": {nm: ctx.engine(i) for i, nm in enumerate(PASS_NAMES)},
+           "kernels": {nm: ctx.kernel(i) for i, nm in enumerate(PASS_NAMES)},
            "sample": f"{k} random genes of the workload (full n={n}), the workload's "
                      f"normed_sum size factors given; fit + theta + bread + Wald per step"}
     fitted = {"genes": genes,
@@ -659,6 +660,7 @@ def main():
         ms = float(t.item())
     value = world * G / (ms / 1e3)
     engines = {name: ctx.engine(k) for k, name in enumerate(PASS_NAMES)}
+    kernels = {name: ctx.kernel(k) for k, name in enumerate(PASS_NAMES)}
     fitted_main = (out["beta"].view(G, p).cpu().numpy(), out["iters"].cpu().numpy(),
                    out["theta"].cpu().numpy())
     off_np = out["off"].cpu().numpy()
@@ -838,7 +840,7 @@ def main():
         "plain": plain,
         "roofline": roof, "cpu_baseline": cpu, "parity": parity, "e2e": e2e, "clocks": clk,
         "gpu_launches": int(launches),
-        "breakdown": {"form": "chosen", "engines": engines, "passes": passes,
+        "breakdown": {"form": "chosen", "engines": engines, "kernels": kernels, "passes": passes,
                       "irls_rescued_genes": rescued,
                       "parallelism": f"genes sharded over {world} rank(s), no exchange during "
                                      f"the fit; p-values all-gathered for BH",

@@ -38,6 +38,7 @@ EXPORTS = (
     "devil_group_order", "devil_ctx_set_profiling", "devil_ctx_profile", "devil_ctx_engine",
     "devil_p_adjust_device_static", "devil_fit_overdispersion_new", "devil_fit_batch",
     "devil_p_adjust_device", "devil_ctx_profile_tc", "devil_ctx_irls_rescued",
+    "devil_ctx_pass_kernel",
 )
 
 
@@ -134,6 +135,8 @@ def load():
         L.devil_ctx_irls_rescued.restype = i64
         L.devil_ctx_engine.argtypes = [vp, i]
         L.devil_ctx_engine.restype = i
+        L.devil_ctx_pass_kernel.argtypes = [vp, i]
+        L.devil_ctx_pass_kernel.restype = C.c_char_p
         L.devil_p_adjust_device_static.argtypes = [i64, vp, i, vp, vp, C.c_char_p, C.c_size_t]
         _lib = L
     return _lib
@@ -194,6 +197,12 @@ class Context:
         "tensor_wide" (IRLS, p = 5..32) or "none"."""
         e = load().devil_ctx_engine(self.h, int(kind))
         return {0: "register", 1: "shared", 2: "groups", 3: "tensor", 4: "tensor_wide"}.get(e, "none")
+
+    def kernel(self, kind: int) -> str:
+        """The kernel of that launch (the names of devil_ctx_pass_kernel): the
+        bread and MOM of continuous designs have kernels of their own, which
+        engine() reports as the per-cell engine of their p."""
+        return load().devil_ctx_pass_kernel(self.h, int(kind)).decode()
 
     def synchronize(self):
         self.check(load().devil_ctx_synchronize(self.h))

@@ -121,6 +121,7 @@ struct devil_ctx {
     double prof_tc_flops[4] = {0, 0, 0, 0};  // tensor-core FLOPs issued (MMA shapes, padding included)
     int64_t irls_rescued = 0;                 // genes the last fit refitted on the CUDA-core engine
     int last_engine[4] = {-1, -1, -1, -1};
+    const char* last_kernel[4] = {"none", "none", "none", "none"};
     // DEVIL_DEBUG: CUDA events at the phase boundaries of a fit
     std::vector<std::pair<const char*, cudaEvent_t>> marks;
     // pinned chunks of large uploads, two per thread (allocated by the first one)
@@ -1318,7 +1319,9 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
     L.plain = plan.plain;
     L.dependent = follows;
     size_t e0 = ctx->profiling ? prof_event(ctx) : 0;
-    // (the FP64 matrix engine is, to callers, the per-cell engine of its p)
+    // (the FP64 matrix engine is, to devil_ctx_engine's callers, the per-cell
+    // engine of its p; devil_ctx_pass_kernel names the kernel)
+    const char*& ran = ctx->last_kernel[kind];
     ctx->last_engine[kind] = (int)(plan.engine != ENGINE_C64 ? plan.engine
                                    : dp.P <= reg_max_p()     ? ENGINE_REG
                                                              : ENGINE_GEN);
@@ -1344,16 +1347,20 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
                                      grp_slices_tile(tiles, gg.S, dp.n, ctx->sm_count),
                                      kind != PASS_IRLS,
                                      ctx->stream, rowexp_fresh));
+            ran = "grp_slices";
         } else {
+            ran = "grp_pass";
             LAUNCH(launch_grp_pass(kind, gg, prm, dp.val_u16, tiles, ctx->stream));
         }
     } else if (plan.engine == ENGINE_REG) {
+        ran = "reg_pass";
         LAUNCH(launch_reg_pass(L));
     } else if (plan.engine == ENGINE_TC) {
         if (!dp.zimg) {
             dp.zimg = ws<float4>(ctx, "tc_zimg", (size_t)tc_zimg_float4s(dp.n));
             LAUNCH(launch_tc_zimg(dp.Xrm, dp.xs, dp.n, dp.P, dp.zimg, ctx->stream));
         }
+        ran = "tc_pass";
         LAUNCH(launch_tc_pass(L, dp.zimg));
     } else if (plan.engine == ENGINE_TCW) {
         if (!dp.tcw_ready) {
@@ -1373,14 +1380,18 @@ void launch_pass(devil_ctx* ctx, const DevProblem& dp, PassKind kind, const Pass
                                       dp.off_f, t, ctx->stream));
             dp.tcw_ready = true;
         }
+        ran = dp.tcw.zimg ? "tcw_pass" : "tcw_pass without image";
         LAUNCH(launch_tcw_pass(L, dp.tcw));
     } else if (plan.engine == ENGINE_C64) {
         L.vec = want_vec;
+        ran = "cell64";
         LAUNCH(launch_cell64_pass(L));
     } else if (kind == PASS_MOM && !plan.plain && mom_cells_supported(dp.P, dp.xs)) {
         // (the shared-memory engine's plan: its runs of cells set the sums)
+        ran = "mom_cells";
         LAUNCH(launch_mom_cells(L, tiles * plan.GT));
     } else {
+        ran = "gen_pass";
         LAUNCH(launch_gen_pass(L));
     }
     if (ctx->profiling) {
@@ -1695,8 +1706,10 @@ void run_irls(devil_ctx* ctx, const DevProblem& dp, double* beta, float* beta_f,
     ctx->irls_rescued = nr;
     if (nr == 0) return;
     const PassPlan p2 = plan_for(PASS_IRLS, dp, form, false);
+    const char* kernel = ctx->last_kernel[PASS_IRLS];
     const int64_t l2 = irls_loop(ctx, dp, p2, beta, beta_f, k, iters, status, max_iter, eps, form, nr);
     ctx->last_engine[PASS_IRLS] = (int)plan.engine;  // the fit's engine (the rescue is counted apart)
+    ctx->last_kernel[PASS_IRLS] = kernel;
     if (ctx->profiling) {
         // the rescue loop's passes: the rescued genes' iteration counts
         int32_t* passes = ws<int32_t>(ctx, "irls_rescue_passes", G);
@@ -2256,6 +2269,11 @@ int devil_ctx_set_profiling(devil_ctx* ctx, int enable) {
 int devil_ctx_engine(const devil_ctx* ctx, int pass_kind) {
     if (!ctx || pass_kind < 0 || pass_kind > 3) return -1;
     return ctx->last_engine[pass_kind];
+}
+
+const char* devil_ctx_pass_kernel(const devil_ctx* ctx, int pass_kind) {
+    if (!ctx || pass_kind < 0 || pass_kind > 3) return "none";
+    return ctx->last_kernel[pass_kind];
 }
 
 int devil_ctx_profile(devil_ctx* ctx, int pass_kind, int64_t* launches, double* ms,

@@ -172,6 +172,11 @@ DEVIL_API int64_t devil_ctx_irls_rescued(const devil_ctx *ctx);
  * p x p contractions as split-TF32 MMAs over a dense count image), -1 none
  * yet. */
 DEVIL_API int devil_ctx_engine(const devil_ctx *ctx, int pass_kind);
+/* The kernel of that launch (no counterpart in the reference): "reg_pass",
+ * "gen_pass", "cell64" (bread/meat on FP64 matrix tiles), "mom_cells" (MOM by
+ * warps; engine 1), "grp_slices", "grp_pass", "tc_pass", "tcw_pass", "tcw_pass
+ * without image", or "none". */
+DEVIL_API const char *devil_ctx_pass_kernel(const devil_ctx *ctx, int pass_kind);
 
 /* ---- full pipeline --------------------------------------------------- */
 /* fit_devil(x, design_matrix, clusters, overdispersion, init_overdispersion,
