@@ -1180,7 +1180,30 @@ bool tcw_mle_wanted(const DevProblem& dp) {
     return dp.precision == DEVIL_PREC_TC_TF32 || dp.P > reg_max_p();
 }
 
-PassPlan plan_engine(PassKind k, const DevProblem& dp, int form, bool allow_tcw = true) {
+// Bread and meat of continuous designs on FP64 matrix tiles (kernels_cell64.cu)?
+// Above eight columns always; below, the register engine spreads a few genes or
+// few cells over more threads, so the tiles need blocks enough (32 genes x a
+// chunk of 1,024 cells, 2,048 to four columns, or a cluster).  Pass, register
+// engine / tiles:
+//   no clusters, p = 4: 300 x 1,500 19 / 78 us, 2,000 x 20,000 (630 blocks) 379 /
+//     428, 1,000 x 100,000 (1,568) 953 / 834, 8,000 x 30,000 2,146 / 1,853
+//   p = 5: 300 x 1,500 (20 blocks) 20 / 58, 300 x 16,000 (160) 83 / 77; p = 8:
+//     300 x 16,000 139 / 97, 8,000 x 30,000 4,880 / 2,391
+//   clusters, p = 8: 40 x 20,000 in 7 (40 blocks) 39 / 41, 64 x 3,000 in 40 (80)
+//     70 / 16, 2,000 x 5,000 in 40 1,950 / 162; p = 3: 500 x 20,000 in 7 105 / 117,
+//     in 40 213 / 117, 2,000 x 5,000 in 7 167 / 119
+// (the register engine's threads idle in clusters of a few hundred cells).
+bool cell64_pays(const devil_ctx* ctx, const DevProblem& dp, int n_clusters) {
+    if (dp.P > reg_max_p()) return true;
+    const int64_t tiles = (dp.G + cell64_tile_genes() - 1) / cell64_tile_genes();
+    const int64_t sm = ctx->sm_count;
+    if (n_clusters <= 0) return tiles * dp.nfine >= (dp.P <= 4 ? 8 : 1) * sm;
+    const int64_t blocks = tiles * std::max<int64_t>(n_clusters, dp.n / 1024);
+    return dp.P <= 4 ? blocks >= sm && dp.n / n_clusters <= 1024 : 2 * blocks >= sm;
+}
+
+PassPlan plan_engine(const devil_ctx* ctx, PassKind k, const DevProblem& dp, int form, bool allow_tcw,
+                     int n_clusters) {
     const int P = dp.P;
     // the plain comparison form: every pass on the per-cell shared-memory
     // engine, FP32 per-cell arithmetic for the FP32 passes (IRLS, MLE)
@@ -1188,9 +1211,7 @@ PassPlan plan_engine(PassKind k, const DevProblem& dp, int form, bool allow_tcw 
     if (dp.grp.active) return {ENGINE_GRP, 1};
     if (k == PASS_IRLS && allow_tcw && tcw_wanted(dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
     if (k == PASS_MLE && allow_tcw && tcw_mle_wanted(dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
-    // bread/meat: FP64 matrix tiles (p = 4, 10,000 x 100,000: 8.5 ms in the
-    // register engine, 7.9 here; below p = 3 the register engine)
-    if (cell64_supported(k, P, dp.xs)) return {ENGINE_C64, cell64_tile_genes()};
+    if (cell64_supported(k, P, dp.xs) && cell64_pays(ctx, dp, n_clusters)) return {ENGINE_C64, cell64_tile_genes()};
     const bool tc = tc_enabled(k) ||
                     (dp.precision == DEVIL_PREC_TC_TF32 && (k == PASS_IRLS || k == PASS_MLE));
     if (P <= tc_max_p() && tc) return {ENGINE_TC, tc_tile_genes(k)};
@@ -1215,8 +1236,9 @@ PassPlan plan_engine(PassKind k, const DevProblem& dp, int form, bool allow_tcw 
     return {ENGINE_GEN, gen_default_gt(k, P)};
 }
 
-PassPlan plan_for(PassKind k, const DevProblem& dp, int form, bool allow_tcw = true) {
-    PassPlan p = plan_engine(k, dp, form, allow_tcw);
+PassPlan plan_for(const devil_ctx* ctx, PassKind k, const DevProblem& dp, int form, bool allow_tcw = true,
+                  int n_clusters = 0) {
+    PassPlan p = plan_engine(ctx, k, dp, form, allow_tcw, n_clusters);
     p.kind = k;
     return p;
 }
@@ -1673,7 +1695,7 @@ void run_irls(devil_ctx* ctx, const DevProblem& dp, double* beta, float* beta_f,
     CK(cudaMemsetAsync(iters, 0, G * sizeof(int32_t), st));
     CK(cudaMemsetAsync(status, 0, G * sizeof(int32_t), st));
     if (G == 0 || max_iter <= 0) return;
-    const PassPlan plan = plan_for(PASS_IRLS, dp, form);
+    const PassPlan plan = plan_for(ctx, PASS_IRLS, dp, form);
     if (plan.GT <= 0) fail(ctx, DEVIL_ERR_UNSUPPORTED, "p = %d unsupported", dp.P);
     const int limit = tcw_rescue_steps(max_iter);
     const bool rescue = plan.engine == ENGINE_TCW;
@@ -1705,7 +1727,7 @@ void run_irls(devil_ctx* ctx, const DevProblem& dp, double* beta, float* beta_f,
     CK(cudaStreamSynchronize(st));
     ctx->irls_rescued = nr;
     if (nr == 0) return;
-    const PassPlan p2 = plan_for(PASS_IRLS, dp, form, false);
+    const PassPlan p2 = plan_for(ctx, PASS_IRLS, dp, form, false);
     const char* kernel = ctx->last_kernel[PASS_IRLS];
     const int64_t l2 = irls_loop(ctx, dp, p2, beta, beta_f, k, iters, status, max_iter, eps, form, nr);
     ctx->last_engine[PASS_IRLS] = (int)plan.engine;  // the fit's engine (the rescue is counted apart)
@@ -1723,7 +1745,7 @@ void run_irls(devil_ctx* ctx, const DevProblem& dp, double* beta, float* beta_f,
 void run_mom(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, const double* beta_d,
              double* theta, int form) {
     if (dp.G == 0) return;
-    const PassPlan plan = plan_for(PASS_MOM, dp, form);
+    const PassPlan plan = plan_for(ctx, PASS_MOM, dp, form);
     int32_t* cnt = nullptr;
     const int32_t* act = all_genes(ctx, dp, &cnt, plan.engine == ENGINE_GRP);  // (mom_finalize maps slots)
     const int tiles = (int)((dp.G + plan.GT - 1) / plan.GT);
@@ -1749,7 +1771,7 @@ void run_mle(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, const do
     cudaStream_t st = ctx->stream;
     const int64_t G = dp.G;
     if (G == 0) return;
-    PassPlan plan = plan_for(PASS_MLE, dp, form);
+    PassPlan plan = plan_for(ctx, PASS_MLE, dp, form);
     if (plan.GT <= 0) fail(ctx, DEVIL_ERR_UNSUPPORTED, "p = %d unsupported for MLE", dp.P);
     MleState s;
     s.x = ws<double>(ctx, "mle_x", G);
@@ -1827,12 +1849,12 @@ void run_sandwich(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, con
                   double* meat, int form) {
     cudaStream_t st = ctx->stream;
     if (dp.G == 0) return;
-    PassPlan plan = plan_for(PASS_SANDWICH, dp, form);
+    PassPlan plan = plan_for(ctx, PASS_SANDWICH, dp, form, true, n_clusters);
     // the grouped sandwich needs the cells keyed by cluster too
     if (plan.engine == ENGINE_GRP && n_clusters > 0 && dp.grp.C != n_clusters) {
         DevProblem plain = dp;
         plain.grp.active = false;
-        plan = plan_for(PASS_SANDWICH, plain, form);
+        plan = plan_for(ctx, PASS_SANDWICH, plain, form, true, n_clusters);
     }
     if (plan.GT <= 0) fail(ctx, DEVIL_ERR_UNSUPPORTED, "p = %d unsupported", dp.P);
     int32_t* cnt = nullptr;
@@ -1881,10 +1903,16 @@ void run_sandwich(devil_ctx* ctx, const DevProblem& dp, const float* beta_f, con
         return;
     }
     // cluster-aligned segments: every cluster block split into pieces of
-    // at most L cells (1-based exclusive ends, R/main.R:193)
+    // at most L cells (1-based exclusive ends, R/main.R:193).  The FP64 matrix
+    // engine has few tiles (32 genes) and walks a piece 32 cells at a time: pieces
+    // that give one wave of blocks, down to 128 cells (1 gene x 50,000 cells in 7
+    // clusters, p = 24: the pass takes 279 us with pieces of 1,024 cells)
     const int64_t n = dp.n;
-    int want = (ctx->sm_count * 2 + tiles - 1) / tiles;
-    int64_t L = std::max<int64_t>(1024, (n + want - 1) / std::max(1, want));
+    const bool c64 = plan.engine == ENGINE_C64;
+    const int occ = c64 ? pass_blocks_per_sm(PASS_SANDWICH, plan.engine, dp.P, plan.GT, dp.val_u16, 0) : 2;
+    int want = (ctx->sm_count * std::max(1, occ) + tiles - 1) / tiles;
+    if (c64) want = std::max(1, want - n_clusters);  // (every cluster's last piece is short)
+    int64_t L = std::max<int64_t>(c64 ? 128 : 1024, (n + want - 1) / std::max(1, want));
     std::vector<int32_t> hb{0};
     std::vector<int32_t> hc;
     int64_t start = 0;

@@ -1,7 +1,8 @@
-// The FP64 per-cell passes of designs of more than eight columns without few
-// distinct rows: bread / per-cluster score sums (src/variance.cpp:22-47,
-// :207-217; PassSandwich of passes.cuh) and MOM moments
-// (src/mom_overdispersion.cpp:34-45; PassMOM, mom_cells_kernel below).
+// The FP64 per-cell passes of designs without few distinct rows: bread /
+// per-cluster score sums (src/variance.cpp:22-47, :207-217; PassSandwich of
+// passes.cuh) above eight columns, and from three where the size gives blocks
+// enough (cell64_pays), and MOM moments above eight (src/mom_overdispersion.cpp:
+// 34-45; PassMOM, mom_cells_kernel below).
 //
 // Bread, per gene and cell: eta = off + x . beta, mu = exp(eta), the weight; then
 // sum_c w_gc x_ci x_cj for every i <= j: a contraction of the weights (genes x
