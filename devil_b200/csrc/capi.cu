@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/devil_b200.h"
+#include "group_cut.h"
 #include "internal.h"
 
 using namespace devil;
@@ -832,53 +833,28 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     // cluster order, so a gene's entries of a slice are too, and a piece is a
     // run of them (f_ptr).
     // Where a search for the dispersion follows (search_follows) the slices are
-    // cut at the clusters too, so that the order of every sum stays.
+    // cut at the clusters too, so that the order of every sum stays; also where
+    // the pieces would not fit the clustered pass's shared memory (2,048 clusters
+    // and two design rows: from 14 M cells).
     std::vector<int64_t> hks(K + 1);
     CK(cudaMemcpyAsync(hks.data(), kst, (K + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    const bool by_cluster = search_follows(overdispersion);
-    std::vector<int32_t> sl_start{0}, sl_key, kslice(U + 1);
-    std::vector<int32_t> f_key, f_base, f_slice, f_loc, f_kslice(K + 1);
-    for (int u = 0; u < U; ++u) {
-        kslice[u] = (int32_t)sl_key.size();
-        const int step = by_cluster ? 1 : C;
-        for (int k = u * C; k < (u + 1) * C; k += step) {
-            const int64_t a = hks[k], cnt = hks[k + step] - a;
-            const int64_t ranges = (cnt + kSliceCells - 1) / kSliceCells;
-            for (int64_t q = 1; q <= ranges; ++q) {
-                sl_start.push_back((int32_t)(a + cnt * q / ranges));
-                sl_key.push_back(u);
-            }
-        }
-    }
-    kslice[U] = (int32_t)sl_key.size();
-    const int NSL = (int)sl_key.size();
+    int smem_max = 0;
+    CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    const SliceCut cut = cut_slices_fitting(
+        hks, U, C, kSliceCells, search_follows(overdispersion),
+        [&](int pieces) { return grp_smem_bytes(PASS_SANDWICH, P, K, pieces) <= (size_t)smem_max - 1024; });
+    const int NSL = (int)cut.sl_key.size(), NF = (int)cut.f_key.size();
     if (NSL < 1 || NSL > kMaxSlices) {
         if (ctx->debug) fprintf(stderr, "devil_b200: design not grouped (%d slices)\n", NSL);
         return;
     }
-    if (C > 1) {
-        int sl = 0;
-        for (int k = 0; k < K; ++k) {
-            f_kslice[k] = (int32_t)f_key.size();
-            for (int64_t a = hks[k]; a < hks[k + 1];) {
-                while (sl_start[sl + 1] <= a) ++sl;  // (no slice is empty)
-                f_key.push_back(k);
-                f_slice.push_back(sl);
-                f_base.push_back(sl_start[sl]);
-                f_loc.push_back((int32_t)(a - sl_start[sl]));
-                a = std::min<int64_t>(hks[k + 1], sl_start[sl + 1]);
-            }
-        }
-        f_kslice[K] = (int32_t)f_key.size();
-    }
-    const int NF = (int)f_key.size();
     int32_t* d_sl_start = ws<int32_t>(ctx, "grp_sl_start", NSL + 1);
     int32_t* d_sl_key = ws<int32_t>(ctx, "grp_sl_key", NSL);
     int32_t* d_kslice = ws<int32_t>(ctx, "grp_kslice", U + 1);
-    h2d(ctx, d_sl_start, sl_start.data(), NSL + 1);
-    h2d(ctx, d_sl_key, sl_key.data(), NSL);
-    h2d(ctx, d_kslice, kslice.data(), U + 1);
+    h2d(ctx, d_sl_start, cut.sl_start.data(), NSL + 1);
+    h2d(ctx, d_sl_key, cut.sl_key.data(), NSL);
+    h2d(ctx, d_kslice, cut.kslice.data(), U + 1);
     int32_t* cslice = ws<int32_t>(ctx, "grp_cslice", n);
     int32_t* cloc = ws<int32_t>(ctx, "grp_cloc", n);
     double* E = ws<double>(ctx, "grp_E", n);  // exp(offset) in slice order
@@ -922,11 +898,11 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
             h2d(ctx, d, v.data(), v.size());
             return d;
         };
-        gr.f_key = up("grp_f_key", f_key);
-        gr.f_base = up("grp_f_base", f_base);
-        gr.f_kslice = up("grp_f_kslice", f_kslice);
-        int32_t* d_f_slice = up("grp_f_slice", f_slice);
-        int32_t* d_f_loc = up("grp_f_loc", f_loc);
+        gr.f_key = up("grp_f_key", cut.f_key);
+        gr.f_base = up("grp_f_base", cut.f_base);
+        gr.f_kslice = up("grp_f_kslice", cut.f_kslice);
+        int32_t* d_f_slice = up("grp_f_slice", cut.f_slice);
+        int32_t* d_f_loc = up("grp_f_loc", cut.f_loc);
         gr.NF = NF;
         gr.f_ptr = ws<int64_t>(ctx, "grp_f_ptr", (size_t)dp.G * (NF + 1));
         LAUNCH(launch_piece_ptr(gent, dp.val_u16, gptr, dp.G, NSL, d_f_slice, d_f_loc, NF, gr.f_ptr, st));

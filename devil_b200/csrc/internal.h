@@ -272,6 +272,8 @@ struct NodArgs {
 };
 cudaError_t launch_new_od(const NodArgs& a, const double* Xcm, double* xcolsum, cudaStream_t st);
 
+// shared memory of a block of that pass (NGq groups, S slices or pieces)
+size_t grp_smem_bytes(PassKind k, int P, int NGq, int S);
 cudaError_t launch_grp_pass(PassKind kind, const GrpGeom& geo, const PassParamsAny& prm, int val_u16,
                             int max_slots, cudaStream_t st);
 // the IRLS, MLE, MOM and bread passes of the design-group engine,
