@@ -901,11 +901,15 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
         gr.f_key = up("grp_f_key", cut.f_key);
         gr.f_base = up("grp_f_base", cut.f_base);
         gr.f_kslice = up("grp_f_kslice", cut.f_kslice);
-        int32_t* d_f_slice = up("grp_f_slice", cut.f_slice);
-        int32_t* d_f_loc = up("grp_f_loc", cut.f_loc);
         gr.NF = NF;
-        gr.f_ptr = ws<int64_t>(ctx, "grp_f_ptr", (size_t)dp.G * (NF + 1));
-        LAUNCH(launch_piece_ptr(gent, dp.val_u16, gptr, dp.G, NSL, d_f_slice, d_f_loc, NF, gr.f_ptr, st));
+        if (cut.by_cluster) {  // every piece is a slice
+            gr.f_ptr = gptr;
+        } else {
+            int32_t* d_f_slice = up("grp_f_slice", cut.f_slice);
+            int32_t* d_f_loc = up("grp_f_loc", cut.f_loc);
+            gr.f_ptr = ws<int64_t>(ctx, "grp_f_ptr", (size_t)dp.G * (NF + 1));
+            LAUNCH(launch_piece_ptr(gent, dp.val_u16, gptr, dp.G, NSL, d_f_slice, d_f_loc, NF, gr.f_ptr, st));
+        }
     }
     dbg_mark(ctx, "g.csr");
     CK(cudaMemcpyAsync(h + 1, bad + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

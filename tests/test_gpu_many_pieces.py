@@ -32,3 +32,18 @@ def test_meat_of_many_clusters(dv):
         # the cluster sums carry the rules' 1e-11 of the sum of the terms' sizes and
         # are not small beside it (counts well off the coefficients): 1e-9
         np.testing.assert_allclose(meat[g], ref, rtol=1e-9)
+
+
+# the same terms summed in another order; the residual sums cancel by at most 1e4
+# and the meat squares them: 1e-10 of the diagonal scale
+def test_meat_of_a_fit_cut_at_the_clusters(dv):
+    """A fit with MLE cuts its slices at the clusters (every piece is a slice), the
+    single step by design row (three pieces a slice)."""
+    from devil_b200 import synthetic
+    P = synthetic.make("binary", seed=3, G=20, n=30000)
+    clusters = np.repeat([1, 2, 3], [8000, 2000, 20000])
+    f = dv.fit_devil((P.rowptr, P.col, P.val, P.n), P.X, clusters=clusters, overdispersion="MLE", size_factors=P.sf_true)
+    meat = dv.compute_clustered_meat(P.X, (P.rowptr, P.col, P.val, P.n), f["beta"], f["overdispersion"], P.sf_true,
+                                     np.array([8000, 10000, 30000], np.int32))
+    d = np.sqrt(np.einsum("gii->gi", meat))
+    assert np.nanmax(np.abs(f["meat"] - meat) / (d[:, :, None] * d[:, None, :])) <= 1e-10
