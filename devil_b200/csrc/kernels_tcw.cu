@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
                 : nullptr;
     bool zlost = false;  // (thread kWW) a bulk copy did not arrive in time
 
-    int issued = 0;   // chunks whose MMAs were committed (uniform)
+    int issued = 0;   // chunks whose MMAs were committed (uniform; after zlost not the last one's)
     int drained = 0;  // runs added into the total (uniform)
     for (int k = 0; k < nchunk; ++k) {
         const int st = k & 1;
@@ -510,12 +510,20 @@ __global__ void __launch_bounds__(kWNT, 1) tcw_pass_kernel(PassGeom geo, PassPar
         issued = k + 1;
     }
     cp_async_wait<0>();
-    // the last commit completes after every MMA of the block; wait for it on
-    // the error path too, so that no MMA is in flight when the tensor memory
-    // is freed
-    if (issued > 0 &&
-        !mbar_wait_bounded(&bars[(issued - 1) & 1], (uint32_t)(((issued - 1) >> 1) & 1)))
+    // No copy may be in flight when the stages are used again or the block ends,
+    // and no MMA when the tensor memory is freed, on the error path too.  Thread
+    // kWW waits for the bulk copy that it has not seen land: the one that it lost,
+    // or, when the loop was left, that of the chunk it was left at (not issued if
+    // this thread's wait had given up: then this one runs out too).
+    if (tid == kWW && tw.zimg && (zlost || issued < nchunk)) {
+        const int z = zlost ? issued - 1 : issued;
+        mbar_wait_bounded(&zbars[z & 1], (uint32_t)((z >> 1) & 1));
         atomicExch(&abort_flag, 1);
+    }
+    // the last commit completes after every MMA (after zlost there is none for the
+    // last chunk: thread kWW waits for the one before, the others' wait runs out)
+    const int last = issued - 1 - (zlost ? 1 : 0);
+    if (last >= 0 && !mbar_wait_bounded(&bars[last & 1], (uint32_t)((last >> 1) & 1))) atomicExch(&abort_flag, 1);
     tc_fence_after();
     __syncthreads();  // abort_flag is final from here on
     const bool good = !abort_flag;
