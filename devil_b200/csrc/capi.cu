@@ -129,8 +129,7 @@ struct devil_ctx {
     char* stage = nullptr;
     cudaEvent_t stage_ev[2 * kStageThreads] = {};
     // contexts of devil_fit_batch's workers between two calls, with their
-    // workspaces (batch_mu: calls of several threads each take their own)
-    std::mutex batch_mu;
+    // workspaces (g_batch_mu: calls of several threads each take their own)
     std::vector<devil_ctx*> batch;
     bool is_worker = false;
 };
@@ -176,13 +175,35 @@ void fail(devil_ctx* ctx, int code, const char* fmt, ...) {
     throw Fail{code};
 }
 
-// gives the idle batch workers' memory back; false when there are none
-bool release_batch(devil_ctx* ctx) {
+// The idle batch workers of every context, whose `batch` lists g_batch_mu guards:
+// any context of the device that runs out of memory gives them back (ws).
+std::mutex g_batch_mu;
+std::vector<devil_ctx*> g_batch_owners;  // the contexts with idle workers
+
+size_t ws_bytes(const devil_ctx* ctx) {
+    size_t held = 0;
+    for (auto& kv : ctx->bufs) held += kv.second.bytes;
+    return held;
+}
+// takes the idle workers of `owner`, or of every context on the device
+std::vector<devil_ctx*> take_idle(devil_ctx* owner, int device) {
     std::vector<devil_ctx*> idle;
-    {
-        std::lock_guard<std::mutex> lk(ctx->batch_mu);
-        idle.swap(ctx->batch);
+    std::lock_guard<std::mutex> lk(g_batch_mu);
+    for (size_t i = 0; i < g_batch_owners.size();) {
+        devil_ctx* o = g_batch_owners[i];
+        if (owner ? o != owner : o->device != device) {
+            ++i;
+            continue;
+        }
+        idle.insert(idle.end(), o->batch.begin(), o->batch.end());
+        o->batch.clear();
+        g_batch_owners.erase(g_batch_owners.begin() + i);
     }
+    return idle;
+}
+// gives their memory back; false when there are none
+bool release_idle(devil_ctx* owner, int device) {
+    const std::vector<devil_ctx*> idle = take_idle(owner, device);
     for (auto* c : idle) devil_ctx_destroy(c);
     return !idle.empty();
 }
@@ -197,7 +218,7 @@ T* ws(devil_ctx* ctx, const std::string& name, size_t count) {
         b.p = nullptr;
         b.bytes = 0;
         cudaError_t e = cudaMalloc(&b.p, bytes);
-        if (e == cudaErrorMemoryAllocation && release_batch(ctx)) {
+        if (e == cudaErrorMemoryAllocation && release_idle(nullptr, ctx->device)) {
             cudaGetLastError();
             e = cudaMalloc(&b.p, bytes);
         }
@@ -2193,17 +2214,25 @@ void read_settings(devil_ctx* ctx) {
     const char* dbg = getenv("DEVIL_DEBUG");
     ctx->debug = (dbg && atoi(dbg)) ? 1 : 0;
 }
-// The workers' contexts after a batch: kept for the next one while their
-// workspaces hold less than 1/64 of the device, until the context ends or runs
-// out of memory; destroyed after an error, or when another call's are kept.
+// The workers' contexts after a batch: kept for the next one while a context's
+// idle workers hold at most kBatchKeep in their workspaces, until it ends or any
+// context on the device runs out of memory; destroyed after an error.  Four
+// problems of about 1,500 genes x 9,000 cells leave 152 MiB; a set that holds
+// more takes far longer than the 30 ms that its allocations cost.
+constexpr size_t kBatchKeep = (size_t)512 << 20;
+constexpr int kBatchWorkers = 8;
 void keep_batch(devil_ctx* ctx, std::vector<devil_ctx*>& wc, bool ok) {
-    size_t held = 0, free_b = 0, total = 0;
-    for (auto* c : wc)
-        for (auto& kv : c->bufs) held += kv.second.bytes;
-    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) ok = false;
-    if (ok && held <= total / 64) {
-        std::lock_guard<std::mutex> lk(ctx->batch_mu);
-        if (ctx->batch.empty()) ctx->batch.swap(wc);
+    if (ok) {
+        std::lock_guard<std::mutex> lk(g_batch_mu);
+        size_t held = 0;
+        for (auto* c : ctx->batch) held += ws_bytes(c);
+        const bool had = !ctx->batch.empty();
+        while (!wc.empty() && (int)ctx->batch.size() < kBatchWorkers && held + ws_bytes(wc.back()) <= kBatchKeep) {
+            held += ws_bytes(wc.back());
+            ctx->batch.push_back(wc.back());
+            wc.pop_back();
+        }
+        if (!had && !ctx->batch.empty()) g_batch_owners.push_back(ctx);
     }
     for (auto* c : wc) devil_ctx_destroy(c);
     wc.clear();
@@ -2237,7 +2266,7 @@ int devil_ctx_create(int device, devil_ctx** out) {
 
 int devil_ctx_destroy(devil_ctx* ctx) {
     if (!ctx) return DEVIL_OK;
-    release_batch(ctx);
+    release_idle(ctx, ctx->device);
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->stage) cudaFreeHost(ctx->stage);
@@ -2354,14 +2383,16 @@ int devil_fit_batch(devil_ctx* ctx, int n_problems, const devil_problem* problem
         return DEVIL_ERR_ARG;
     }
     if (n_problems == 0) return DEVIL_OK;
-    workers = std::max(1, std::min(std::min(workers, 8), n_problems));
+    workers = std::max(1, std::min(std::min(workers, kBatchWorkers), n_problems));
     // the workers' contexts of the call before, and new ones: creating one and
     // growing its workspaces is a hundred allocations and frees (four problems of
-    // about 1,500 genes: 49 ms with new contexts, 17 with kept ones)
-    std::vector<devil_ctx*> wc;
-    {
-        std::lock_guard<std::mutex> lk(ctx->batch_mu);
-        wc.swap(ctx->batch);
+    // about 1,500 genes: 49 ms with new contexts, 17 with kept ones); those beyond
+    // this call's workers stay idle
+    std::vector<devil_ctx*> wc = take_idle(ctx, ctx->device);
+    if ((int)wc.size() > workers) {
+        std::vector<devil_ctx*> rest(wc.begin() + workers, wc.end());
+        wc.resize(workers);
+        keep_batch(ctx, rest, true);
     }
     for (auto* c : wc) read_settings(c);
     while ((int)wc.size() < workers) {
