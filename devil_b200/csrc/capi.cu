@@ -208,6 +208,15 @@ bool release_idle(devil_ctx* owner, int device) {
     return !idle.empty();
 }
 
+size_t idle_bytes(int device) {
+    size_t held = 0;
+    std::lock_guard<std::mutex> lk(g_batch_mu);
+    for (auto* o : g_batch_owners)
+        if (o->device == device)
+            for (auto* c : o->batch) held += ws_bytes(c);
+    return held;
+}
+
 // grow-only named device workspace
 template <class T>
 T* ws(devil_ctx* ctx, const std::string& name, size_t count) {
@@ -648,11 +657,18 @@ void prepare_cells(devil_ctx* ctx, DevProblem& dp) {
 
 // whether the wide tensor-core engine's dense count image fits half of the
 // free device memory (asked once per fit, and only where that engine could
-// run: the query costs milliseconds on a busy device)
-bool tcw_fits(const DevProblem& dp) {
+// run: the query costs milliseconds on a busy device).  What this context holds
+// for these images, and what idle batch workers hold, counts as free: a fit takes
+// the same engine the second time as the first.
+bool tcw_fits(const devil_ctx* ctx, const DevProblem& dp) {
     if (dp.tcw_fits < 0) {
         size_t fr = 0, tot = 0;
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = 0;
+        for (const char* name : {"tcw_y", "tcw_xt", "tcw_off", "tcw_z"}) {
+            const auto it = ctx->bufs.find(name);
+            if (it != ctx->bufs.end()) fr += it->second.bytes;
+        }
+        fr += idle_bytes(ctx->device);
         const double need = (double)dp.G * tcw_npad(dp.n) * (dp.val_u16 ? 2.0 : 4.0) +
                             (double)(dp.xs + 1) * tcw_npad(dp.n) * 4.0;
         dp.tcw_fits = need <= 0.5 * (double)fr ? 1 : 0;
@@ -1165,8 +1181,8 @@ struct PassPlan {
 // the DEVIL_PREC_TC_TF32 precision and, by default, from p = 9 on, where
 // the alternative is the FP64 shared-memory engine (about 20x slower per
 // IRLS pass at p = 16 and 32 on the 20,000 x 100,000 continuous workload)
-bool tcw_wanted(const DevProblem& dp) {
-    if (!tcw_supported(dp.P, dp.xs) || !tcw_fits(dp)) return false;
+bool tcw_wanted(const devil_ctx* ctx, const DevProblem& dp) {
+    if (!tcw_supported(dp.P, dp.xs) || !tcw_fits(ctx, dp)) return false;
     const char* e = getenv("DEVIL_TCW");
     if (e && *e) return atoi(e) == 1;
     return dp.precision == DEVIL_PREC_TC_TF32 || dp.P > reg_max_p();
@@ -1174,8 +1190,8 @@ bool tcw_wanted(const DevProblem& dp) {
 // its dispersion (MLE) pass: DEVIL_TCW_MLE=1 / 0; otherwise as the IRLS
 // pass (the FP64 shared-memory pass it replaces from p = 9 on is about 13x
 // slower on the 20,000 x 100,000 continuous workload at p = 16 and 32)
-bool tcw_mle_wanted(const DevProblem& dp) {
-    if (!tcw_supported(dp.P, dp.xs) || !tcw_fits(dp)) return false;
+bool tcw_mle_wanted(const devil_ctx* ctx, const DevProblem& dp) {
+    if (!tcw_supported(dp.P, dp.xs) || !tcw_fits(ctx, dp)) return false;
     const char* e = getenv("DEVIL_TCW_MLE");
     if (e && *e) return atoi(e) == 1;
     return dp.precision == DEVIL_PREC_TC_TF32 || dp.P > reg_max_p();
@@ -1210,8 +1226,8 @@ PassPlan plan_engine(const devil_ctx* ctx, PassKind k, const DevProblem& dp, int
     // engine, FP32 per-cell arithmetic for the FP32 passes (IRLS, MLE)
     if (form == DEVIL_FORM_PLAIN) return {ENGINE_GEN, gen_default_gt(k, P), k, 1};
     if (dp.grp.active) return {ENGINE_GRP, 1};
-    if (k == PASS_IRLS && allow_tcw && tcw_wanted(dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
-    if (k == PASS_MLE && allow_tcw && tcw_mle_wanted(dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
+    if (k == PASS_IRLS && allow_tcw && tcw_wanted(ctx, dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
+    if (k == PASS_MLE && allow_tcw && tcw_mle_wanted(ctx, dp)) return {ENGINE_TCW, tcw_tile_genes(k)};
     if (cell64_supported(k, P, dp.xs) && cell64_pays(ctx, dp, n_clusters)) return {ENGINE_C64, cell64_tile_genes()};
     const bool tc = tc_enabled(k) ||
                     (dp.precision == DEVIL_PREC_TC_TF32 && (k == PASS_IRLS || k == PASS_MLE));

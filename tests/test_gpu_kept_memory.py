@@ -60,3 +60,24 @@ def test_idle_batch_workers_are_given_back(dv, own):
         del fill
         ctx.close()
     assert _free() > b - (64 << 20)  # (the workers are gone)
+
+
+def test_a_second_fit_takes_the_same_engine(dv, own):
+    """A wide continuous fit whose count image (4 GB) just fits half of the free
+    memory: the first call's images are the second call's."""
+    import torch
+    G, n, p = 4000, 500000, 9
+    rng = np.random.default_rng(3)
+    X = np.column_stack([np.ones(n), rng.normal(size=(n, p - 1))])
+    cols = [np.unique(rng.integers(0, n, 400)).astype(np.int32) for _ in range(G)]
+    ptr = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int64)
+    x = (ptr, np.concatenate(cols), np.ones(int(ptr[-1]), np.uint16), n)
+    run = lambda: dv.fit_devil(x, X, overdispersion=False, max_iter=2)["beta"]
+    fill = torch.empty(_free() - (11 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        first = run()
+        assert own.kernel(0) == "tcw_pass"
+        np.testing.assert_array_equal(run(), first)
+        assert own.kernel(0) == "tcw_pass"
+    finally:
+        del fill
