@@ -659,7 +659,8 @@ void prepare_cells(devil_ctx* ctx, DevProblem& dp) {
 // free device memory (asked once per fit, and only where that engine could
 // run: the query costs milliseconds on a busy device).  What this context holds
 // for these images, and what idle batch workers hold, counts as free: a fit takes
-// the same engine the second time as the first.
+// the same engine the second time as the first.  DEVIL_TCW_IMAGE=0 leaves the
+// products' image out.
 bool tcw_fits(const devil_ctx* ctx, const DevProblem& dp) {
     if (dp.tcw_fits < 0) {
         size_t fr = 0, tot = 0;
@@ -673,7 +674,8 @@ bool tcw_fits(const devil_ctx* ctx, const DevProblem& dp) {
                             (double)(dp.xs + 1) * tcw_npad(dp.n) * 4.0;
         dp.tcw_fits = need <= 0.5 * (double)fr ? 1 : 0;
         // (with the products' image when that fits too)
-        dp.tcw_zfits = need + (double)tcw_zimg_bytes(dp.P, dp.n) <= 0.5 * (double)fr;
+        const char* e = getenv("DEVIL_TCW_IMAGE");
+        dp.tcw_zfits = !(e && *e && atoi(e) == 0) && need + (double)tcw_zimg_bytes(dp.P, dp.n) <= 0.5 * (double)fr;
     }
     return dp.tcw_fits == 1;
 }
