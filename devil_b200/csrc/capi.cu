@@ -307,7 +307,8 @@ bool stage_ready(devil_ctx* ctx) {
     return true;
 }
 
-// Host to device on the context's stream; the source may be reused on return.
+// Host to device on the context's stream.  A pageable source may be reused on
+// return; a pinned one must stay as it is until the stream is synchronised.
 // Large pageable arrays are cut into chunks that threads take in turn: fill a
 // pinned chunk, queue its copy, and fill the thread's other chunk meanwhile (a
 // chunk is filled again only after its event).  80 MB: 7.3 ms by one pageable

@@ -19,7 +19,6 @@ namespace devil {
 DEV void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 DEV void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 
-
 constexpr float kLog2e = 1.4426950408889634f;
 
 // MUFU.EX2 / MUFU.RCP through PTX (approximate, ~1-2 ulp; FTZ).
@@ -56,39 +55,10 @@ DEV float load_val(const uint16_t* v, int64_t e) { return (float)__ldg(v + e); }
 DEV float load_val(const float* v, int64_t e) { return __ldg(v + e); }
 
 // ---------------------------------------------------------------------
-// small dense FP64 linear algebra on column-major p x p matrices held by
-// one thread (local memory / registers).  LU with partial pivoting, the
-// factorisation Eigen's MatrixXd::inverse() uses for dynamic sizes.
-// Returns false when a pivot is exactly zero or not finite.
+// solution of a p x p system by one thread, column-major, from its LU
+// factors with partial pivoting (row swaps piv), the factorisation Eigen's
+// MatrixXd::inverse() uses for dynamic sizes
 // ---------------------------------------------------------------------
-DEV bool lu_factor(int p, double* A, int* piv) {
-    bool ok = true;
-    for (int k = 0; k < p; ++k) {
-        int mx = k;
-        double mv = fabs(A[k * p + k]);
-        for (int i = k + 1; i < p; ++i) {
-            double v = fabs(A[k * p + i]);
-            if (v > mv) { mv = v; mx = i; }
-        }
-        piv[k] = mx;
-        if (mx != k)
-            for (int j = 0; j < p; ++j) {
-                double t = A[j * p + k];
-                A[j * p + k] = A[j * p + mx];
-                A[j * p + mx] = t;
-            }
-        double d = A[k * p + k];
-        if (!(d != 0.0) || !isfinite(d)) ok = false;
-        double rd = 1.0 / d;
-        for (int i = k + 1; i < p; ++i) {
-            double l = A[k * p + i] * rd;
-            A[k * p + i] = l;
-            for (int j = k + 1; j < p; ++j) A[j * p + i] -= l * A[j * p + k];
-        }
-    }
-    return ok;
-}
-
 DEV void lu_solve(int p, const double* LU, const int* piv, double* x) {
     for (int k = 0; k < p; ++k)
         if (piv[k] != k) { double t = x[k]; x[k] = x[piv[k]]; x[piv[k]] = t; }
@@ -101,15 +71,6 @@ DEV void lu_solve(int p, const double* LU, const int* piv, double* x) {
         double s = x[i];
         for (int j = i + 1; j < p; ++j) s -= LU[j * p + i] * x[j];
         x[i] = s / LU[i * p + i];
-    }
-}
-
-// inverse of an LU-factored matrix into Ainv (column-major)
-DEV void lu_inverse(int p, const double* LU, const int* piv, double* Ainv) {
-    for (int c = 0; c < p; ++c) {
-        double* x = Ainv + c * p;
-        for (int i = 0; i < p; ++i) x[i] = (i == c) ? 1.0 : 0.0;
-        lu_solve(p, LU, piv, x);
     }
 }
 
