@@ -1511,9 +1511,9 @@ const int32_t* all_genes(devil_ctx* ctx, const DevProblem& dp, int32_t** count_o
 // the active genes: grp_slices_tile.)  On the first
 // loop of a shape bucket (pass kind, engine, p, count type, log2 n,
 // log2 G, half-octaves of the density) in this process, each candidate
-// plan runs the loop's first pass once untimed and three times timed (CUDA
-// events on the context stream, all genes active); the fastest is kept for the
-// bucket.  The candidates' FP32 segment sums can round differently (well
+// plan runs the loop's first pass once untimed and once timed, close ones three
+// times timed (CUDA events on the context stream, all genes active); the fastest is
+// kept for the bucket.  The candidates' FP32 segment sums can round differently (well
 // inside the parity bars).  DEVIL_AUTOTUNE=0 keeps the
 // heuristic defaults.
 struct TuneKey {
@@ -1568,11 +1568,20 @@ PassPlan autotune(devil_ctx* ctx, const DevProblem& dp, const PassPlan& base, co
         cudaEvent_t t0, t1;
         CK(cudaEventCreate(&t0));
         CK(cudaEventCreate(&t1));
-        // once untimed, then the fastest of three rounds over the candidates in
-        // turn: with one run each a clock step could pick the plan
+        // once untimed, then once timed; candidates within a tenth of the fastest
+        // run twice more, in turn, as with one run each a clock step could pick the
+        // plan (a first pass takes 4 ms at 8,500 x 30,000, p = 16, MLE: the first fit
+        // of a shape pays for every run)
         std::vector<float> ms(cands.size(), INFINITY);
-        for (int rep = 0; rep < 4; ++rep)
+        std::vector<char> on(cands.size(), 1);
+        for (int rep = 0; rep < 4; ++rep) {
+            if (rep == 2) {
+                const float close = 1.1f * *std::min_element(ms.begin(), ms.end());
+                for (size_t i = 0; i < cands.size(); ++i) on[i] = ms[i] <= close;
+                if (std::count(on.begin(), on.end(), 1) < 2) break;
+            }
             for (size_t i = 0; i < cands.size(); ++i) {
+                if (!on[i]) continue;
                 const PassPlan& pl = cands[i];
                 const int tiles = (int)((n0 + pl.GT - 1) / pl.GT);
                 const int nseg = choose_nseg(ctx, dp, pl, tiles, form);
@@ -1586,6 +1595,7 @@ PassPlan autotune(devil_ctx* ctx, const DevProblem& dp, const PassPlan& base, co
                 CK(cudaEventElapsedTime(&t, t0, t1));
                 if (rep > 0) ms[i] = std::min(ms[i], t);
             }
+        }
         float best_ms = 0.f;
         for (size_t i = 0; i < cands.size(); ++i) {
             // a candidate replaces the default only when clearly faster
