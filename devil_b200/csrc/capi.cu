@@ -1183,7 +1183,10 @@ struct PassPlan {
 // selects it wherever it applies, DEVIL_TCW=0 never; otherwise it runs for
 // the DEVIL_PREC_TC_TF32 precision and, by default, from p = 9 on, where
 // the alternative is the FP64 shared-memory engine (about 20x slower per
-// IRLS pass at p = 16 and 32 on the 20,000 x 100,000 continuous workload)
+// IRLS pass at p = 16 and 32 on the 20,000 x 100,000 continuous workload).
+// Below, the register engine is faster over a fit of that workload (IRLS + MLE,
+// register / tensor cores): p = 5 122 + 75 / 195 + 205 ms, p = 6 144 + 130 / 199 +
+// 212, p = 8 244 + 159 / 202 + 213.
 bool tcw_wanted(const devil_ctx* ctx, const DevProblem& dp) {
     if (!tcw_supported(dp.P, dp.xs) || !tcw_fits(ctx, dp)) return false;
     const char* e = getenv("DEVIL_TCW");

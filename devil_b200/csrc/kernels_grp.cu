@@ -479,10 +479,13 @@ __global__ void __launch_bounds__(kOffNT) seg_offsets_kernel(const int64_t* rowp
 constexpr int kSegTile = 2048;   // entries per round of a block
 constexpr int kSegNT = 256;
 // The line between the two: 32 neighbouring entries of a row have about as many
-// keys as the design has rows.  With 2 rows (4,000 x 1 M, 408 M entries) the warp
-// kernel takes 1.0 ms and this one 2.3; with 62 rows it loses as above; their cost
-// per entry meets near 24.  Above 1,024 keys a tile holds fewer than two entries
-// per key: no runs to write.
+// keys as the design has rows, and each key costs the warp kernel a step.  Warp
+// kernel / this one, 1,000 x 1 M, 100 M entries: 16-bit counts 0.45 / 0.74 ms at 2
+// rows, 0.58 / 0.73 at 8, 0.74 / 0.74 at 16, 0.81 / 0.77 at 24, 1.00 / 0.74 at 64;
+// float counts 0.77 / 0.78 at 12, 0.95 / 0.78 at 24; 4,000 x 100,000, 20 M: 0.21 /
+// 0.22 at 20, 0.23 / 0.22 at 24.  Above 1,024 keys a tile holds fewer than two
+// entries per key: no runs to write.  (Five blocks an SM hold a thread to 48
+// registers, about 48 bytes of it spilled.)
 constexpr int kSegRowsMin = 24;
 constexpr int kSegKeysMax = 1024;
 
