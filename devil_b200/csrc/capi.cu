@@ -312,8 +312,12 @@ bool stage_ready(devil_ctx* ctx) {
 // Large pageable arrays are cut into chunks that threads take in turn: fill a
 // pinned chunk, queue its copy, and fill the thread's other chunk meanwhile (a
 // chunk is filled again only after its event).  80 MB: 7.3 ms by one pageable
-// copy, 3.6 here.  Batch workers already upload side by side and keep to plain
-// copies, as do pinned and device sources.
+// copy, 3.6 here.  A thread per 16 chunks, two at least: starting a thread costs as
+// much as several chunks, and one that reads another core's cache is slow (one
+// copy / a thread per 4 chunks / per 16, ms, caches warm: 8 MB 0.73 / 0.90 / 0.68,
+// 16 MB 1.20 / 1.57 / 1.04, 24 MB 1.61 / 1.89 / 1.41, 32 MB 2.08 / 2.14 / 1.83; from
+// memory 16 MB 1.88 / 1.73 / 1.19, 32 MB 3.42 / 2.33 / 1.88).  Batch workers already
+// upload side by side and keep to plain copies, as do pinned and device sources.
 void upload_bytes(devil_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!bytes) return;
     cudaPointerAttributes at{};
@@ -347,7 +351,7 @@ void upload_bytes(devil_ctx* ctx, void* dst, const void* src, size_t bytes) {
         }
     };
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
-    const int nt = (int)std::min<size_t>(std::min<size_t>(kStageThreads, cores), (chunks + 3) / 4);
+    const int nt = (int)std::min<size_t>(std::min<size_t>(kStageThreads, cores), std::max<size_t>(2, (chunks + 15) / 16));
     std::vector<std::thread> th;
     try {
         th.reserve(kStageThreads);

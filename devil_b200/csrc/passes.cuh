@@ -574,7 +574,7 @@ DEV void reg_pass_body(PassGeom geo, typename Pass::Params prm) {
         // gene tile works on the current one (one row ahead left most of an L2
         // round trip exposed); with one column, one cell ahead: the second row's
         // registers would change the blocks per SM, and with them the segments
-        // that the sums are cut into
+        // that the FP32 sums are cut into
         constexpr int D = P == 1 ? 1 : 2;
         float xn[D][P];
         float on[D] = {};
