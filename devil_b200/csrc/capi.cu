@@ -893,12 +893,18 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
         if (ctx->debug) fprintf(stderr, "devil_b200: design not grouped (%d slices)\n", NSL);
         return;
     }
-    int32_t* d_sl_start = ws<int32_t>(ctx, "grp_sl_start", NSL + 1);
-    int32_t* d_sl_key = ws<int32_t>(ctx, "grp_sl_key", NSL);
-    int32_t* d_kslice = ws<int32_t>(ctx, "grp_kslice", U + 1);
-    h2d(ctx, d_sl_start, cut.sl_start.data(), NSL + 1);
-    h2d(ctx, d_sl_key, cut.sl_key.data(), NSL);
-    h2d(ctx, d_kslice, cut.kslice.data(), U + 1);
+    // (one upload for all of the cut's lists)
+    std::vector<int32_t> lists;
+    auto put = [&](const std::vector<int32_t>& v) {
+        lists.insert(lists.end(), v.begin(), v.end());
+        return lists.size() - v.size();
+    };
+    const size_t at_start = put(cut.sl_start), at_key = put(cut.sl_key), at_kslice = put(cut.kslice);
+    const size_t at_fkey = put(cut.f_key), at_fbase = put(cut.f_base), at_fkslice = put(cut.f_kslice);
+    const size_t at_fslice = put(cut.f_slice), at_floc = put(cut.f_loc);
+    int32_t* d_lists = ws<int32_t>(ctx, "grp_cut", lists.size());
+    h2d(ctx, d_lists, lists.data(), lists.size());
+    int32_t* d_sl_start = d_lists + at_start;
     int32_t* cslice = ws<int32_t>(ctx, "grp_cslice", n);
     int32_t* cloc = ws<int32_t>(ctx, "grp_cloc", n);
     double* E = ws<double>(ctx, "grp_E", n);  // exp(offset) in slice order
@@ -937,22 +943,16 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
                             gptr, gent, st));
     if (NF > 0) {
         auto& gr = dp.grp;
-        auto up = [&](const char* nm, const std::vector<int32_t>& v) {
-            int32_t* d = ws<int32_t>(ctx, nm, v.size());
-            h2d(ctx, d, v.data(), v.size());
-            return d;
-        };
-        gr.f_key = up("grp_f_key", cut.f_key);
-        gr.f_base = up("grp_f_base", cut.f_base);
-        gr.f_kslice = up("grp_f_kslice", cut.f_kslice);
+        gr.f_key = d_lists + at_fkey;
+        gr.f_base = d_lists + at_fbase;
+        gr.f_kslice = d_lists + at_fkslice;
         gr.NF = NF;
         if (cut.by_cluster) {  // every piece is a slice
             gr.f_ptr = gptr;
         } else {
-            int32_t* d_f_slice = up("grp_f_slice", cut.f_slice);
-            int32_t* d_f_loc = up("grp_f_loc", cut.f_loc);
             gr.f_ptr = ws<int64_t>(ctx, "grp_f_ptr", (size_t)dp.G * (NF + 1));
-            LAUNCH(launch_piece_ptr(gent, dp.val_u16, gptr, dp.G, NSL, d_f_slice, d_f_loc, NF, gr.f_ptr, st));
+            LAUNCH(launch_piece_ptr(gent, dp.val_u16, gptr, dp.G, NSL, d_lists + at_fslice, d_lists + at_floc, NF, gr.f_ptr,
+                                    st));
         }
     }
     dbg_mark(ctx, "g.csr");
@@ -1115,8 +1115,8 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     g.gent = gent;
     g.gptr = gptr;
     g.sl_start = d_sl_start;
-    g.sl_key = d_sl_key;
-    g.kslice = d_kslice;
+    g.sl_key = d_lists + at_key;
+    g.kslice = d_lists + at_kslice;
     g.rs = rs;
     g.rw = rw;
     g.rm = rm;
