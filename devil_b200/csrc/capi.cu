@@ -915,14 +915,13 @@ void build_groups(devil_ctx* ctx, DevProblem& dp, const int32_t* ends_host, int 
     double* rs = ws<double>(ctx, "grp_rs", (size_t)nrules * kRuleCap);
     double* rw = ws<double>(ctx, "grp_rw", (size_t)nrules * kRuleCap);
     int32_t* rm = ws<int32_t>(ctx, "grp_rm", nrules);
-    double* scr = ws<double>(ctx, "grp_scr", (size_t)4 * n);
     double* rerr = ws<double>(ctx, "grp_rerr", nrules);
     // (a search: the rules' sums in one order whatever the group sizes, as for the slices)
     const bool one_block = search_follows(overdispersion);
-    LAUNCH(launch_group_rules(permC, gsC, U, dp.off, n, scr, rs, rw, rm, rerr, bad + 1, one_block, st));
-    if (C > 1)  // rules U.. : the (row, cluster) groups
-        LAUNCH(launch_group_rules(permF, gsF, K, dp.off, n, scr, rs + (size_t)U * kRuleCap,
-                                  rw + (size_t)U * kRuleCap, rm + U, rerr + U, bad + 1, one_block, st));
+    const int n_fine = C > 1 ? K : 0;  // rules U.. : the (row, cluster) groups
+    double* scr = ws<double>(ctx, "grp_scr", group_rules_scratch(n, U, n_fine, one_block));
+    LAUNCH(launch_group_rules(permC, gsC, U, permF, gsF, n_fine, dp.off, n, scr, rs, rw, rm, rerr, bad + 1, one_block,
+                              st));
     dbg_mark(ctx, "g.rules");
     // CSR copy ordered by slice within each gene: 4-byte entries (index in
     // the slice, 16-bit count) or 8-byte ones for float counts

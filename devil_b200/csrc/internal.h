@@ -319,11 +319,14 @@ cudaError_t launch_fine_keys(const int32_t* ucell, const int32_t* ends, int C, i
 cudaError_t launch_group_starts(const int32_t* ks, int64_t n, int K, int64_t* gstart,
                                 cudaStream_t st);
 cudaError_t launch_exp(const double* x, int64_t n, double* y, cudaStream_t st);
-// the rules of the groups perm[gs[b]..gs[b+1]) (cells sorted by offset within
-// a group); scr: 4 n doubles
-cudaError_t launch_group_rules(const int32_t* perm, const int64_t* gs, int nrules, const double* off, int64_t n,
-                               double* scr, double* rs, double* rw, int32_t* rm, double* rerr,
-                               int32_t* bad, bool one_block, cudaStream_t st);
+// the rules of the groups perm1[gs1[b]..gs1[b+1]) (cells sorted by offset within
+// a group), b < n1, then those of the n2 groups of perm2; scr: group_rules_scratch
+// doubles
+size_t group_rules_scratch(int64_t n, int n1, int n2, bool one_block);
+cudaError_t launch_group_rules(const int32_t* perm1, const int64_t* gs1, int n1, const int32_t* perm2,
+                               const int64_t* gs2, int n2, const double* off, int64_t n, double* scr, double* rs,
+                               double* rw, int32_t* rm, double* rerr, int32_t* bad, bool one_block,
+                               cudaStream_t st);
 cudaError_t launch_gather_keys(const int32_t* keys, const int32_t* cells, int64_t n, int32_t* out,
                                cudaStream_t st);
 int group_csr_segment(int64_t nnz, int64_t G, int K);  // entries per segment
