@@ -632,7 +632,7 @@ void prepare_design(devil_ctx* ctx, DevProblem& dp, const double* X, int P, bool
     }
     dp.stats = ws<double>(ctx, "stats", (size_t)dp.G * 6);
     LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.nnz, dp.n, dp.stats,
-                             ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), st));
+                             ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), st, dp.gorder));
 }
 
 // what the per-cell engines read besides the counts: the design by cell and
@@ -2619,7 +2619,7 @@ int devil_estimate_dispersion(devil_ctx* ctx, const devil_counts* counts,
         upload_counts(ctx, counts, dp);
         dp.stats = ws<double>(ctx, "stats", (size_t)dp.G * 6);
         LAUNCH(launch_gene_stats(dp.rowptr, dp.val, dp.val_u16, dp.G, dp.nnz, dp.n, dp.stats,
-                                 ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), ctx->stream));
+                                 ws<char>(ctx, "gene_sums", gene_sums_bytes(dp.G)), ctx->stream, dp.gorder));
         upload_offsets(ctx, dp, offset_vector);
         double* th = ws<double>(ctx, "theta0", dp.G);
         float* k = ws<float>(ctx, "k", dp.G);

@@ -358,10 +358,13 @@ cudaError_t launch_x_rowmajor(const double* Xcm, int64_t n, int P, int xs, float
 cudaError_t launch_x_rowmajor_d(const double* Xcm, int64_t n, int P, int xs, double* Xrm,
                                 cudaStream_t st);
 cudaError_t launch_double_to_float(const double* in, float* out, int64_t m, cudaStream_t st);
-// stats: G x 6; sums: gene_sums_bytes(G) of scratch (uint16 counts)
+// stats: G x 6; sums: gene_sums_bytes(G) of scratch (uint16 counts); order: the
+// genes in the order the warps of a row each take them, largest first (null: gene
+// order)
 size_t gene_sums_bytes(int64_t G);
 cudaError_t launch_gene_stats(const int64_t* rowptr, const void* val, int val_u16, int64_t G, int64_t nnz,
-                              int64_t n, double* stats, void* sums, cudaStream_t st);
+                              int64_t n, double* stats, void* sums, cudaStream_t st,
+                              const int32_t* order = nullptr);
 // (colsum_u32, n: zeroed scratch of n cells; normed_sum of 16-bit counts
 // then sums with 32-bit integer atomics)
 cudaError_t launch_colstats(const int64_t* rowptr, const int32_t* col, const void* val,

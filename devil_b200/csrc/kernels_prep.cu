@@ -172,37 +172,47 @@ cudaError_t launch_x_rowmajor_d(const double* Xcm, int64_t n, int P, int xs, dou
 // stats[g*6 + 0..5] = mean, sample variance (n-1), sum y,
 //                     sum (y-1) y, max y, nnz
 // ------------------------------------------------------------------
-__global__ void gene_stats_kernel(const int64_t* rowptr, const float* val, int64_t G, int64_t n,
-                                  double* stats) {
+// (order: the genes in the order the warps take them, largest first; null: gene
+// order)
+template <class VT>
+__global__ void gene_stats_kernel(const int64_t* rowptr, const VT* val, int64_t G, int64_t n,
+                                  double* stats, const int32_t* order) {
     int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (g >= G) return;
+    if (order) g = order[g];
     const int64_t e0 = rowptr[g], e1 = rowptr[g + 1];
-    // Float counts that are whole numbers: one pass with exact integer sums
-    // of y and y^2 (below 2^64 for any int32 cell count and counts below 2^16)
-    // and the variance from the exact numerator n sum y^2 - (sum y)^2 in 128
-    // bits, so a uint16 (gene_sums_kernel) and a float copy of the same counts
-    // give the same statistics.  Other counts: a second pass over the squared
+    // Counts that are whole numbers (always for uint16; checked for float): one
+    // pass with exact integer sums of y and y^2 (below 2^64 for any int32 cell
+    // count and counts below 2^16) and the variance from the exact numerator n sum
+    // y^2 - (sum y)^2 in 128 bits, so a uint16 (here or in gene_sums_kernel) and a
+    // float copy of the same counts give the same statistics.  Other counts: a second pass over the squared
     // deviations in FP64.
     unsigned long long s1 = 0, s2 = 0;
     double s = 0.0, mx = 0.0;
     bool whole = true;
     constexpr int U = 4;  // loads in flight per lane
     for (int64_t base = e0 + lane; base < e1; base += 32 * U) {
-        float raw[U];
+        VT raw[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) raw[u] = base + 32 * u < e1 ? __ldg(val + base + 32 * u) : 0.f;
+        for (int u = 0; u < U; ++u) raw[u] = base + 32 * u < e1 ? __ldg(val + base + 32 * u) : VT(0);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const double y = (double)raw[u];
-            s += y;
             mx = fmax(mx, y);
-            const bool w = y >= 0.0 && y < 65536.0 && y == floor(y);
-            whole = whole && w;
-            if (w) {
-                const unsigned long long v = (unsigned long long)y;
+            if constexpr (std::is_same<VT, uint16_t>::value) {
+                const unsigned long long v = (unsigned long long)raw[u];
                 s1 += v;
                 s2 += v * v;
+            } else {
+                s += y;
+                const bool w = y >= 0.0 && y < 65536.0 && y == floor(y);
+                whole = whole && w;
+                if (w) {
+                    const unsigned long long v = (unsigned long long)y;
+                    s1 += v;
+                    s2 += v * v;
+                }
             }
         }
     }
@@ -368,19 +378,30 @@ __global__ void gene_stats_from_sums_kernel(const int64_t* rowptr, const GeneSum
 
 size_t gene_sums_bytes(int64_t G) { return (size_t)G * sizeof(GeneSums); }
 
+// Rows of at most kShortRows cells: a warp per row (20,000 genes x 500 cells, 15
+// entries a row: 14 us, 34 by spans; 2,000 x 4,000, 600 entries: 15 us, 18; 2,000 x
+// 8,000, 2,400 entries: 25, 17; 300 x 16,000: 43, 13).
+constexpr int64_t kShortRows = 4096;
 cudaError_t launch_gene_stats(const int64_t* rowptr, const void* val, int val_u16, int64_t G, int64_t nnz,
-                              int64_t n, double* stats, void* sums, cudaStream_t st) {
+                              int64_t n, double* stats, void* sums, cudaStream_t st, const int32_t* order) {
     if (G == 0) return cudaSuccess;
     if (!val_u16) {
-        gene_stats_kernel<<<nblk(G, 8), 256, 0, st>>>(rowptr, (const float*)val, G, n, stats);
+        gene_stats_kernel<float><<<nblk(G, 8), 256, 0, st>>>(rowptr, (const float*)val, G, n, stats, order);
+        return cudaGetLastError();
+    }
+    if (n <= kShortRows) {
+        gene_stats_kernel<uint16_t><<<nblk(G, 8), 256, 0, st>>>(rowptr, (const uint16_t*)val, G, n, stats, order);
         return cudaGetLastError();
     }
     GeneSums* acc = static_cast<GeneSums*>(sums);
     cudaError_t e = cudaMemsetAsync(acc, 0, gene_sums_bytes(G), st);
     if (e != cudaSuccess) return e;
-    // about 64 warps per SM in flight, 1,024 to 16,384 entries each
+    // about 64 warps per SM in flight, up to 16,384 entries each and no fewer than
+    // two rows' or 1,024: a row costs a warp about a microsecond however short it
+    // is (20,000 genes x 100,000 cells, 30 entries a row: 51 us with 1,024, 31 so)
     int64_t span = (nnz / (148 * 64) + 255) / 256 * 256;
-    span = std::max<int64_t>(1024, std::min<int64_t>(16384, span));
+    const int64_t least = std::max<int64_t>(32, std::min<int64_t>(1024, (2 * nnz / G + 7) / 8 * 8));
+    span = std::max<int64_t>(least, std::min<int64_t>(16384, span));
     const unsigned b = nblk((nnz + span - 1) / span, 8);
     if (b > 0) {
         if ((reinterpret_cast<uintptr_t>(val) & 15) == 0)
@@ -602,31 +623,40 @@ DEV double strided_sum(int64_t n, F&& at) {
 // method 1 = normed_sum (R/size_factors.R:75-88), 2 = psinorm (:100-117).
 // The logarithms on every SM, then one block for their sum (in a fixed order),
 // then the division and the offsets on every SM: one block for all of it took
-// 1.29 ms at a million cells, the three take 0.25 ms.
-__global__ void sf_log_kernel(int method, int64_t G, int64_t n, const double* colsum, const double* collog,
-                              const int32_t* colcnt, const int32_t* colmin_bits, double* sf, double* lg,
-                              int32_t* err) {
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (int64_t)gridDim.x * blockDim.x) {
+// 1.29 ms at a million cells, the three take 0.25 ms.  Up to kOneBlock cells one
+// block does all three, with the same sums: there the launches cost more.
+constexpr int64_t kOneBlock = 16384;
+struct SfArgs {
+    int method;
+    int64_t G, n;
+    const double *colsum, *collog;
+    const int32_t *colcnt, *colmin_bits;
+    double offset;
+    double *sf, *off;  // (off holds the logarithms first)
+    float* off_f;
+    int32_t* err;
+};
+DEV void sf_logs(const SfArgs& a, int64_t first, int64_t step) {
+    for (int64_t c = first; c < a.n; c += step) {
         double v;
-        if (G <= 1) {
+        if (a.G <= 1) {
             v = 1.0;
-        } else if (method == 1) {
-            v = colsum[c];
-            if (v == 0.0) *err = 1;
+        } else if (a.method == 1) {
+            v = a.colsum[c];
+            if (v == 0.0) *a.err = 1;
         } else {
-            double m = colcnt[c] < G ? 0.0 : (double)__int_as_float(colmin_bits[c]);
-            v = collog[c] / (double)G - m;
+            double m = a.colcnt[c] < a.G ? 0.0 : (double)__int_as_float(a.colmin_bits[c]);
+            v = a.collog[c] / (double)a.G - m;
         }
-        sf[c] = v;
-        lg[c] = log(v);
+        a.sf[c] = v;
+        a.off[c] = log(v);
     }
 }
-__global__ void __launch_bounds__(1024) sf_mean_kernel(int64_t G, int64_t n, const double* lg, double* gm) {
-    __shared__ double red[32], red2[32];
+// the geometric mean, by one block; valid in thread 0
+DEV double sf_mean(const SfArgs& a, double* red, double* red2) {
     double cntv = 0.0;
-    double acc = strided_sum(n, [&](int64_t c) {
-        const double l = lg[c];
+    double acc = strided_sum(a.n, [&](int64_t c) {
+        const double l = a.off[c];
         const bool ok = !isnan(l);
         cntv += ok ? 1.0 : 0.0;
         return ok ? l : 0.0;
@@ -635,34 +665,57 @@ __global__ void __launch_bounds__(1024) sf_mean_kernel(int64_t G, int64_t n, con
     cntv = warp_sum(cntv);
     if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = acc; red2[threadIdx.x >> 5] = cntv; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0, k = 0.0;
+    double s = 0.0, k = 0.0;
+    if (threadIdx.x == 0)
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { s += red[w]; k += red2[w]; }
-        *gm = (G <= 1) ? 1.0 : exp(s / k);
+    return a.G <= 1 ? 1.0 : exp(s / k);
+}
+DEV void sf_scale(const SfArgs& a, double gm, int64_t first, int64_t step) {
+    for (int64_t c = first; c < a.n; c += step) {
+        double v = (a.G <= 1) ? 1.0 : a.sf[c] / gm;
+        a.sf[c] = v;
+        double o = a.offset + log(v);
+        a.off[c] = o;
+        a.off_f[c] = (float)o;
     }
 }
-__global__ void sf_scale_kernel(int64_t G, int64_t n, const double* gm_p, double offset, double* sf, double* off,
-                                float* off_f) {
-    const double gm = *gm_p;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        double v = (G <= 1) ? 1.0 : sf[c] / gm;
-        sf[c] = v;
-        double o = offset + log(v);
-        off[c] = o;
-        off_f[c] = (float)o;
-    }
+__global__ void sf_log_kernel(SfArgs a) {
+    sf_logs(a, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+__global__ void __launch_bounds__(1024) sf_mean_kernel(SfArgs a, double* gm) {
+    __shared__ double red[32], red2[32];
+    const double m = sf_mean(a, red, red2);
+    if (threadIdx.x == 0) *gm = m;
+}
+__global__ void sf_scale_kernel(SfArgs a, const double* gm) {
+    sf_scale(a, *gm, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+__global__ void __launch_bounds__(1024) sf_block_kernel(SfArgs a) {
+    __shared__ double red[32], red2[32], gm;
+    if (threadIdx.x == 0) *a.err = 0;
+    __syncthreads();
+    sf_logs(a, threadIdx.x, blockDim.x);
+    __syncthreads();
+    const double m = sf_mean(a, red, red2);
+    if (threadIdx.x == 0) gm = m;
+    __syncthreads();
+    sf_scale(a, gm, threadIdx.x, blockDim.x);
 }
 cudaError_t launch_sf_finalize(int method, int64_t G, int64_t n, const double* colsum,
                                const double* collog, const int32_t* colcnt,
                                const int32_t* colmin_bits, double offset, double* sf,
                                double* off, float* off_f, double* gm, int32_t* err, cudaStream_t st) {
+    const SfArgs a{method, G, n, colsum, collog, colcnt, colmin_bits, offset, sf, off, off_f, err};
+    if (n <= kOneBlock) {
+        sf_block_kernel<<<1, 1024, 0, st>>>(a);
+        return cudaGetLastError();
+    }
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int32_t), st);
     if (e != cudaSuccess) return e;
     const unsigned b = (unsigned)std::min<int64_t>(nblk(n, 256), 148 * 8);
-    sf_log_kernel<<<b, 256, 0, st>>>(method, G, n, colsum, collog, colcnt, colmin_bits, sf, off, err);
-    sf_mean_kernel<<<1, 1024, 0, st>>>(G, n, off, gm);
-    sf_scale_kernel<<<b, 256, 0, st>>>(G, n, gm, offset, sf, off, off_f);
+    sf_log_kernel<<<b, 256, 0, st>>>(a);
+    sf_mean_kernel<<<1, 1024, 0, st>>>(a, gm);
+    sf_scale_kernel<<<b, 256, 0, st>>>(a, gm);
     return cudaGetLastError();
 }
 
@@ -693,17 +746,19 @@ cudaError_t launch_sf_given(const double* sf_in, int64_t n, double offset, int u
 // (src/beta.cpp:25-28: theta_0 arrives as float, 1.0/k stored as float).
 // ------------------------------------------------------------------
 // eoff = exp(off), evaluated on every SM beforehand (this kernel's one block
-// took 0.53 ms for a million cells, the two take 0.14 ms)
+// took 0.53 ms for a million cells, the two take 0.14 ms); up to kOneBlock cells
+// null: evaluated here
 __global__ void exp_off_kernel(const double* off, int64_t n, double* eoff) {
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
          c += (int64_t)gridDim.x * blockDim.x)
         eoff[c] = exp(off[c]);
 }
-__global__ void __launch_bounds__(1024) theta0_kernel(const double* stats, const double* eoff, int64_t G, int64_t n,
-                                                      int has_init, double init_value, double* theta0, float* k) {
+__global__ void __launch_bounds__(1024) theta0_kernel(const double* stats, const double* off, const double* eoff,
+                                                      int64_t G, int64_t n, int has_init, double init_value,
+                                                      double* theta0, float* k) {
     __shared__ double red[32];
     __shared__ double moi_s;
-    double acc = strided_sum(n, [&](int64_t c) { return eoff[c]; });
+    double acc = strided_sum(n, [&](int64_t c) { return eoff ? eoff[c] : exp(off[c]); });
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
@@ -732,8 +787,11 @@ cudaError_t launch_theta0(const double* stats, const double* off, int64_t G, int
                           int has_init, double init_value, double* eoff, double* theta0, float* k,
                           cudaStream_t st) {
     if (has_init) n = 0;  // theta_0 is given: no mean of exp(off)
-    if (n > 0) exp_off_kernel<<<(unsigned)std::min<int64_t>(nblk(n, 256), 148 * 8), 256, 0, st>>>(off, n, eoff);
-    theta0_kernel<<<1, 1024, 0, st>>>(stats, eoff, G, n, has_init, init_value, theta0, k);
+    if (n <= kOneBlock)
+        eoff = nullptr;
+    else
+        exp_off_kernel<<<(unsigned)std::min<int64_t>(nblk(n, 256), 148 * 8), 256, 0, st>>>(off, n, eoff);
+    theta0_kernel<<<1, 1024, 0, st>>>(stats, off, eoff, G, n, has_init, init_value, theta0, k);
     return cudaGetLastError();
 }
 
@@ -1089,7 +1147,9 @@ cudaError_t launch_validate_csr(const int64_t* rowptr, const int32_t* col, int64
                                 int64_t nnz, int32_t* bad, cudaStream_t st) {
     if (G == 0) return cudaSuccess;
     const bool vec = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
-    const unsigned b = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nblk(std::max(nnz / 16, G), 256), 148 * 8));
+    // (with short rows more threads: the searches of a thread's row starts follow
+    // one another)
+    const unsigned b = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nblk(std::max(nnz / 16, 4 * G), 256), 148 * 8));
     if (vec)
         validate_csr_kernel<true><<<b, 256, 0, st>>>(rowptr, col, G, n, nnz, bad);
     else
