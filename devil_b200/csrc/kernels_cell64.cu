@@ -37,10 +37,12 @@
 // 18..22 it then spills about 88 bytes; with one block and no spill, 4,000 x
 // 50,000, p = 18 takes 5.5 ms instead of 4.8.
 //
-// Bound by the FP64 pipe: exp and the terms, about 45 operations a gene-cell,
-// and p (p + 1) / 2 multiply-adds.  The engine it replaces kept one output per
-// thread and read two shared doubles per multiply-add.  Measured, 8,500 genes x
-// 30,000 cells, p = 16: bread 42.5 -> 4.8 ms, MOM 19.0 -> 1.6 ms.
+// Bound by the FP64 tensor pipe and the latency around it: at 4,000 x 20,000, p =
+// 16 (two blocks of 122 registers per SM) that pipe is 49 % busy, 65 % with 40
+// clusters, issue slots 45 %, and warps wait for it, for shared memory and at the
+// two barriers of a chunk.  The engine it replaces kept one output per thread and
+// read two shared doubles per multiply-add.  Measured, 8,500 genes x 30,000 cells,
+// p = 16: bread 42.5 -> 4.9 ms, MOM 19.0 -> 1.6 ms.
 #include "internal.h"
 #include "tc_common.cuh"
 
