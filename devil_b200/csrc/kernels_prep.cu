@@ -923,8 +923,12 @@ cudaError_t launch_xtx_inverse(const double* Xcm, int64_t n, int P, double* part
 // beta_0 = (log1p(mean y), 0, ..., 0).  U entries a lane are in flight and are
 // added in order; the genes with the most entries are taken first (one entry at
 // a time, a gene seen in every cell held its warp for 3,000 dependent rounds:
-// 10,000 x 100,000, p = 4: 3.59 -> 2.18 ms).
-template <class VT, int PMAX>
+// 10,000 x 100,000, p = 4: 3.59 -> 2.18 ms).  Up to kShortInit cells one entry a
+// lane (SHORT): rows of a few rounds cost the deep loop its registers and masked
+// loads (p = 4, short / deep: 20,000 x 500 24 / 69 us, 8,000 x 2,000 41 / 58, 6,000 x
+// 3,000 55 / 61, 5,000 x 4,000 78 / 64; p = 12: 65 / 101, 78 / 91, 87 / 101, 114 / 108).
+constexpr int64_t kShortInit = 3072;
+template <class VT, int PMAX, bool SHORT>
 __global__ void init_beta_kernel(const int64_t* rowptr, const int32_t* col, const VT* val,
                                  const double* Xrm, int xs, const double* inv_sf,
                                  const double* ginv, const double* stats, int64_t G, int64_t n,
@@ -944,8 +948,8 @@ __global__ void init_beta_kernel(const int64_t* rowptr, const int32_t* col, cons
     double r[PMAX];
 #pragma unroll
     for (int i = 0; i < PMAX; ++i) r[i] = 0.0;
-    constexpr int U = PMAX <= 8 ? 8 : 4;    // entries in flight
-    constexpr int V = PMAX <= 4 ? 8 : (PMAX <= 8 ? 4 : (PMAX <= 16 ? 2 : 1));  // design rows in flight
+    constexpr int U = SHORT ? 1 : (PMAX <= 8 ? 8 : 4);    // entries in flight
+    constexpr int V = SHORT ? 1 : (PMAX <= 4 ? 8 : (PMAX <= 8 ? 4 : (PMAX <= 16 ? 2 : 1)));  // design rows in flight
     const int64_t e1 = rowptr[g + 1];
     int cn[U];
     VT vn[U];
@@ -1015,15 +1019,16 @@ cudaError_t launch_init_beta(const int64_t* rowptr, const int32_t* col, const vo
         inv_exp_kernel<<<(unsigned)std::min<int64_t>(nblk(n, 256), 1024), 256, 0, st>>>(off, n, inv_sf);
     }
     const unsigned b = nblk(G, 8);
-#define DEVIL_INIT(PM)                                                                          \
-    if (val_u16)                                                                                 \
-        init_beta_kernel<uint16_t, PM><<<b, 256, 0, st>>>(rowptr, col, (const uint16_t*)val, Xrm, \
-                                                            xs, inv_sf, ginv, stats, G, n, P,     \
-                                                            rough, beta, beta_f, order);         \
-    else                                                                                         \
-        init_beta_kernel<float, PM><<<b, 256, 0, st>>>(rowptr, col, (const float*)val, Xrm, xs,   \
-                                                         inv_sf, ginv, stats, G, n, P, rough,     \
-                                                         beta, beta_f, order);
+    auto go = [&](auto kern, auto* v) {
+        kern<<<b, 256, 0, st>>>(rowptr, col, v, Xrm, xs, inv_sf, ginv, stats, G, n, P, rough, beta, beta_f, order);
+    };
+#define DEVIL_INIT(PM)                                                                            \
+    if (val_u16)                                                                                  \
+        go(n <= kShortInit ? init_beta_kernel<uint16_t, PM, true> : init_beta_kernel<uint16_t, PM, false>, \
+           (const uint16_t*)val);                                                                 \
+    else                                                                                          \
+        go(n <= kShortInit ? init_beta_kernel<float, PM, true> : init_beta_kernel<float, PM, false>, \
+           (const float*)val);
     if (P <= 4) {
         DEVIL_INIT(4)
     } else if (P <= 8) {
@@ -1143,12 +1148,38 @@ __global__ void __launch_bounds__(256) validate_csr_kernel(const int64_t* rowptr
     }
     if (b) atomicOr(bad, 1);
 }
+// The same check, a warp a row, for matrices of up to kShortRows cells: their rows
+// end within a few rounds, where the scan searches the row pointers once a row and
+// waits for each load of a search (rows / scan: 20,000 genes x 500 cells 9 / 22 us,
+// 10,000 x 1,500 12 / 20, 6,000 x 3,000 15 / 19, 5,000 x 4,000 19 / 18).
+__global__ void __launch_bounds__(256) validate_rows_kernel(const int64_t* rowptr, const int32_t* col, int64_t G,
+                                                            int64_t n, int64_t nnz, int32_t* bad) {
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    int b = 0;
+    for (int64_t g = warp; g < G; g += nw) {
+        const int64_t e0 = rowptr[g], e1 = rowptr[g + 1];
+        if (e0 < 0 || e1 < e0 || e1 > nnz || (g == G - 1 && e1 != nnz)) {
+            b = 1;
+            continue;
+        }
+        for (int64_t e = e0 + lane; e < e1; e += 32) {
+            const int c = __ldg(col + e), before = e > e0 ? __ldg(col + e - 1) : -1;
+            b |= (c < 0) | (c >= n) | (before >= c);
+        }
+    }
+    if (b) atomicOr(bad, 1);
+}
 cudaError_t launch_validate_csr(const int64_t* rowptr, const int32_t* col, int64_t G, int64_t n,
                                 int64_t nnz, int32_t* bad, cudaStream_t st) {
     if (G == 0) return cudaSuccess;
+    if (n <= kShortRows) {
+        validate_rows_kernel<<<(unsigned)std::min<int64_t>(nblk(G, 8), 148 * 8), 256, 0, st>>>(rowptr, col, G, n,
+                                                                                              nnz, bad);
+        return cudaGetLastError();
+    }
     const bool vec = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
-    // (with short rows more threads: the searches of a thread's row starts follow
-    // one another)
     const unsigned b = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nblk(std::max(nnz / 16, 4 * G), 256), 148 * 8));
     if (vec)
         validate_csr_kernel<true><<<b, 256, 0, st>>>(rowptr, col, G, n, nnz, bad);
